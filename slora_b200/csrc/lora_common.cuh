@@ -89,6 +89,7 @@ struct TileInfo {
   int xrcap;
   bool xok;
   int tok[kTileTokens];  // the entry's token ids (valid when xok)
+  int xscale;            // the entry's scale word (valid when xok)
 };
 
 // Tensor-parallel link of a pipelined shrink (writes its result into every rank's delta buffer and signals) or expand
@@ -118,6 +119,25 @@ struct TpLink {
                //    refill is a whole kernel ahead of the next write.  `half` is not used.
 };
 
+// Division by a launch constant as one multiplication and a shift (n < 2^31).  A 64-bit division costs a producer warp
+// several hundred cycles, and a launch's first copies wait for its first divisions: the producers of the pipelined
+// kernels use none.
+struct FastDiv {
+  uint32_t mul;
+  uint32_t shift;
+  uint32_t d;
+  __device__ __forceinline__ int div(int n) const {
+    return static_cast<int>((static_cast<uint64_t>(static_cast<uint32_t>(n)) * mul) >> shift);
+  }
+};
+// mul = floor(2^(31 + s) / d) + 1 with s = ceil(log2 d): the error of mul is at most 1, that of n * mul below 2^31, which
+// moves the quotient by less than 1 / d.
+inline FastDiv make_fast_div(uint32_t d) {
+  uint32_t s = 0;
+  while ((uint64_t(1) << s) < d) ++s;
+  return FastDiv{static_cast<uint32_t>((uint64_t(1) << (31 + s)) / d + 1), 31 + s, d};
+}
+
 struct ShrinkArgs {
   TileSrc src;
   Tables tb;
@@ -132,6 +152,8 @@ struct ShrinkArgs {
   int delta_width;
   int rank_mult;     // A rows per slot row (1 in the reference layout; N when a rank holds [r, h_in / N] slices)
   int max_rb;        // row blocks enumerated per (tile, projection)
+  FastDiv per_tile;      // pipelined kernel: items enumerated per tile (padded enumeration)
+  FastDiv rows_per_row;  // pipelined kernel: A rows per pool row
   int rows_per_cta;  // <= kMaxRows
   int tok_pass;      // simple kernel: tokens staged per pass
   int piece;         // simple kernel: elements per bulk copy
@@ -159,7 +181,9 @@ struct ExpandArgs {
   int64_t delta_part_stride;
   int rank_mult;
   int max_rank;  // widest rank the delta buffers hold (delta_width * delta_parts): wider adapters are refused
-  int piece;  // elements per bulk copy (power of two dividing pool_stride, <= kChunk)
+  int piece;  // simple kernel: elements per bulk copy (power of two dividing pool_stride, <= kChunk)
+  FastDiv per_tile;  // pipelined kernel: items enumerated per tile (padded enumeration)
+  FastDiv stride;    // pipelined kernel: elements per pool row
   int mma_stage_bytes;  // tensor-core kernel: bytes of one operand tile [128 x kpad_max]
   TpLink tp;
   int32_t* status;
@@ -315,6 +339,7 @@ __device__ __forceinline__ bool lookup_tile(const TileSrc& s, const Tables& tb, 
     if (t.xt != nullptr) {
       k0 = reinterpret_cast<const int4*>(t.xt)[0];
       k1 = reinterpret_cast<const int4*>(t.xt)[1];
+      t.xscale = t.xt[8];
     }
     t.tok[0] = k0.x, t.tok[1] = k0.y, t.tok[2] = k0.z, t.tok[3] = k0.w;
     t.tok[4] = k1.x, t.tok[5] = k1.y, t.tok[6] = k1.z, t.tok[7] = k1.w;
@@ -339,6 +364,7 @@ __device__ __forceinline__ bool lookup_tile(const TileSrc& s, const Tables& tb, 
   t.perm = nullptr;
   t.xt = nullptr;
   t.xrcap = 0;
+  t.xscale = 0;
   t.xok = false;
   if (s.mode == MODE_TOKEN) {
     if (tile_idx >= s.T) return false;

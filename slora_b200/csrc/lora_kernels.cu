@@ -569,6 +569,18 @@ int64_t pipe_grid(int64_t items, int per_tile, bool exact) {
   return grid;
 }
 
+// Adapter rows of a pipelined shrink item.  The more rows an item has, the less often the tile's tokens are staged again
+// (once per item); the fewer items there are, the less evenly they fall on the CTAs.  Sixteen rows where tiles hold
+// several tokens and even the launch's upper bound of tiles leaves eight items a CTA, eight where it leaves four, else
+// four.
+int shrink_item_rows(int64_t T, int64_t slots, int nproj, int delta_width) {
+  const int64_t grid = static_cast<int64_t>(sm_count()) * kPipeCtasPerSm;
+  auto items = [&](int rows) { return slots * nproj * ((delta_width + rows - 1) / rows); };
+  if (delta_width > 8 && T >= 2 * slots && items(16) >= 8 * grid) return 16;
+  if (delta_width > 4 && items(8) >= 4 * grid) return 8;
+  return 4;
+}
+
 int run_shrink(const TileSrc& src, const Tables& tb, const void* w, const void* x, int64_t x_stride, int h_in,
                int nproj, const int* qkvo, void* const* delta, int64_t delta_stride, int delta_width, int dtype,
                unsigned flags, int32_t* status, cudaStream_t stream, const TpLink* tp = nullptr, int rank_mult = 1) {
@@ -687,20 +699,22 @@ int run_shrink(const TileSrc& src, const Tables& tb, const void* w, const void* 
     // runs: neither writes what the other reads before its grid-dependency wait, and their outputs are disjoint
     if (mma_stream == stream) flags |= SLORA_FLAG_PDL;
   }
-  const bool can_pipe = (S % h_in == 0);
+  const bool can_pipe = (S % h_in == 0) && tb.pool_rows < (int64_t(1) << 31);
   const KernelChoice choice = kernel_choice();
   if ((choice == CHOOSE_PIPELINED || tp) && !can_pipe)
     return fail(SLORA_ERR_SHAPE, "No suitable kernel. pipelined shrink needs pool_stride %% h_in == 0");
   if (tp && choice == CHOOSE_SIMPLE) return fail(SLORA_ERR_SHAPE, "No suitable kernel. the linked shrink is pipelined only");
   if (can_pipe && choice != CHOOSE_SIMPLE) {
-    a.rows_per_cta = kMaxRows;
     a.src.xoff = src.xoff;
     a.src.xrcap = src.xrcap;
-    a.max_rb = (delta_width + kMaxRows - 1) / kMaxRows;
+    a.rows_per_cta = shrink_item_rows(src.T, src.slots, nproj, delta_width);
+    a.max_rb = (delta_width + a.rows_per_cta - 1) / a.rows_per_cta;
+    a.per_tile = make_fast_div(static_cast<uint32_t>(nproj * a.max_rb));
+    a.rows_per_row = make_fast_div(static_cast<uint32_t>(S / h_in));
     const int64_t items = static_cast<int64_t>(src.slots) * nproj * a.max_rb;
     const bool exact = (flags & SLORA_FLAG_EXACT_ITEMS) != 0 && src.mode == MODE_PLAN;
     const int64_t grid = pipe_grid(items, nproj * a.max_rb, exact);
-    const size_t smem = kRingBytes;
+    const size_t smem = kShrinkRingBytes;
     auto go = [&](auto k, int which) {
       const int rc2 = ensure_dyn_smem(k, which, smem);
       return rc2 ? rc2 : launch(k, grid, kPipeThreads, smem, flags, stream, a, "shrink(pipelined)");
@@ -830,8 +844,7 @@ int run_expand(const TileSrc& src, const Tables& tb, const void* w, const void* 
     a.src.mma_max_rows = delta_width < kMmaMaxRank ? delta_width : kMmaMaxRank;
     if (mma_stream == stream) flags |= SLORA_FLAG_PDL;  // as in the shrink
   }
-  const int pipe_piece = pow2_divisor(tb.pool_stride, kPipeChunk);
-  bool can_pipe = delta_parts == 1 && delta_stride % 8 == 0 && pipe_piece * kMaxPieces >= kPipeChunk &&
+  bool can_pipe = delta_parts == 1 && delta_stride % 8 == 0 && tb.pool_rows < (int64_t(1) << 31) &&
                   tb.pool_stride < (int64_t(1) << 30) &&
                   (kPipeChunk - 1) / tb.pool_stride + 2 <= kSpanRows;
   for (int p = 0; p < nproj; ++p)
@@ -842,10 +855,11 @@ int run_expand(const TileSrc& src, const Tables& tb, const void* w, const void* 
                                  "plain delta layout");
   if (tp && choice == CHOOSE_SIMPLE) return fail(SLORA_ERR_SHAPE, "No suitable kernel. the linked expand is pipelined only");
   if (can_pipe && choice != CHOOSE_SIMPLE) {
-    a.piece = pipe_piece;
     a.src.xoff = src.xoff;
     a.src.xrcap = src.xrcap;
     set_chunks(kPipeChunk);
+    a.per_tile = make_fast_div(static_cast<uint32_t>(a.chunk_begin[nproj]));
+    a.stride = make_fast_div(static_cast<uint32_t>(tb.pool_stride));
     const int64_t items = static_cast<int64_t>(src.slots) * a.chunk_begin[nproj];
     const bool exact = (flags & SLORA_FLAG_EXACT_ITEMS) != 0 && src.mode == MODE_PLAN;
     const int64_t grid = pipe_grid(items, a.chunk_begin[nproj], exact);

@@ -1,37 +1,43 @@
 // Persistent, warp-specialised, mbarrier-pipelined LoRA shrink / expand kernels (the fast path).
 //
-// Two CTAs per SM (a grid of 2 x SM count) walk their share of the work items (item i belongs to CTA
-// i mod gridDim.x).  The first
-// kProducerWarps warps are producers: the 32 lanes of each resolve 32 upcoming items in parallel (tile record ->
-// table entries -> row addresses and token ids), then feed a ring of shared-memory stages with bulk asynchronous
-// copies (cp.async.bulk + mbarrier complete_tx).  With more than one producer all run the same deterministic
-// allocation and stage g is issued by producer g mod kProducerWarps (measured: no gain on B200 while the consumers
-// are the bottleneck, so one producer is configured).  The remaining warps are consumers: they wait on a stage's "full" barrier, do the arithmetic and release the
-// stage through its "empty" barrier.  Consumer warps never wait for each other (shrink: each warp owns a K-slice and
-// the last warp to finish an item, elected by an atomic counter, adds the partial sums; expand: each warp owns a
-// 1024-element span of the B chunk), so every wait in the kernel is an mbarrier wait with a time limit.
+// Two CTAs per SM (a grid of 2 x SM count) walk their share of the work items (item i belongs to CTA i mod gridDim.x).
+// Two producer warps feed a ring of shared-memory stages with bulk asynchronous copies (cp.async.bulk + mbarrier
+// complete_tx): the lanes of the first resolve 32 upcoming items in parallel (tile record -> table entries -> pool rows
+// and token ids), then both run the same deterministic allocation, the first copying adapter rows and the second
+// activations (after a CTA's first stages also some of the rows).  Eight consumer warps wait on a stage's "full" barrier,
+// do the arithmetic (mma.sync, lora_warp_mma.cuh) and release the stage through its "empty" barrier.  Consumer warps
+// never wait for each other (shrink: each warp owns a K-slice and the last warp to finish an item, elected by an atomic
+// counter, adds the partial sums; expand: each warp owns a 2048-element span of the B chunk).  Every wait is an mbarrier
+// wait with a time limit, but for the meetings of the two producers, each of which only has such waits in between.
 //
-// What shapes the ring (measured on B200): a cp.async.bulk warp-instruction costs the issuing warp 400-600 cycles
-// whatever its size and however many lanes take part, and ~1 us passes before the bytes land.  So a stage is filled
-// by ONE bulk instruction in which every participating lane carries one copy (adapter rows and activation rows
-// alike), stages are made as large as the work item allows (tens of KB), and they are packed back to back in a
-// byte ring of kRingBytes so that several are in flight whatever their size.
+// What bounds a launch (measured on B200, clock64 around the phases of every warp): a stage's round trip - a consumer's
+// release, the producers' reaction, the copies' issue, memory, the consumers - with two or three stages of 34 to 49 KB
+// per CTA in flight.  What it is made of, and what was done about it:
+// * A bulk copy's operands are uniform registers: a warp issues its lanes' copies one after the other, 52 cycles each with
+//   the SM to itself and 75 to 140 beside working consumers.  So copies are few and large (one per pool row that a B
+//   chunk touches, not one per power-of-two piece: 18 -> 6 copies a stage at row stride 5120) and two warps issue.
+// * Divisions: a 64-bit one costs hundreds of cycles, and a stage had five.  The producers use FastDiv and shifts: the
+//   expand's producer time per stage 3300 -> 1900 cycles (q,k,v expand of the 13B-shaped batch 83.8 -> 69.2 us).
+// * Consumers on the tensor pipe: a stage of eight tokens at rank 64 took 3150 cycles of FMA and shuffles, now 1750
+//   (q,k,v expand of the 70B-shaped batch 77.6 -> 55.1 us); the shrink's accumulators became one C fragment whatever the
+//   item's size, so that an item can have sixteen rows and its tokens are staged a quarter as often (208 -> 106 us).
+// * Copies per worker warp with cp.async instead (every consumer its own ring of 4 KB stages, no producers) were correct
+//   and slower, 343 against 216 us per layer of the 13B-shaped batch: the addresses of 16-byte copies and the ring's
+//   bookkeeping are then paid per 4 KB.
 //
-// Programmatic dependent launch: the producer issues the adapter-row copies of the first stages (rows that no kernel
-// on the stream writes) before it executes griddepcontrol.wait and stashes the activation copies (x, y, delta) of
-// those stages; they go out right after the wait.  With a ring of 96 KB two CTAs fit on an SM: in steady state both
-// belong to the running kernel (twice the stages in flight and twice the consumer warps per SM; measured 15 % to
-// 38 % less time per layer than one CTA per SM), and as CTAs of the running kernel retire the next kernel's CTAs
-// take their place and run their prologue under this kernel's tail.
+// Programmatic dependent launch: the first producer copies the adapter rows of the first stages (rows that no kernel on
+// the stream writes) before griddepcontrol.wait; the second waits for the grid right before its first activation copy.
+// Two CTAs fit on an SM: in steady state both belong to the running kernel, and as CTAs of the running kernel retire the
+// next kernel's CTAs take their place and run their prologue under this kernel's tail.
 //
-// Shrink stage  = one item (tile, projection, block of <= 4 rows), or a K-chunk of it when the item exceeds
-//                 kMaxStageBytes: [nrows adapter-row chunks][n token-row chunks]; accumulators stay in registers
-//                 across the chunks of an item.
+// Shrink stage  = one item (tile, projection, block of 4, 8 or 16 rows), or a K-chunk of it when the item exceeds
+//                 kMaxStageBytes: [adapter-row chunks][token-row chunks]; sums stay in registers across the chunks.
 // Expand stage  = one item (tile, projection, 16384-element chunk of B): [B chunk][n y segments][n delta rows].
-//                 y is read through the stage and written back with plain coalesced stores.
+//                 y is read through the stage and written back with plain vector stores.
 #pragma once
 
 #include "lora_common.cuh"
+#include "lora_warp_mma.cuh"
 
 namespace slora {
 
@@ -40,9 +46,14 @@ constexpr int kSlots = 8;  // stage descriptors (barrier pairs) in flight
 #define SLORA_RING_KB 96
 #endif
 #ifndef SLORA_STAGE_KB
-#define SLORA_STAGE_KB 48
+#define SLORA_STAGE_KB 49
 #endif
-constexpr int kRingBytes = SLORA_RING_KB * 1024;  // ring + control block stay below half an SM's shared memory
+#ifndef SLORA_SHRINK_RING_KB
+#define SLORA_SHRINK_RING_KB 98
+#endif
+// ring + control block (+ the shrink's reduction buffers) stay below half an SM's shared memory
+constexpr int kRingBytes = SLORA_RING_KB * 1024;
+constexpr int kShrinkRingBytes = SLORA_SHRINK_RING_KB * 1024;
 #ifndef SLORA_EXPAND_RING_KB
 #define SLORA_EXPAND_RING_KB 104
 #endif
@@ -52,16 +63,17 @@ constexpr int kRingBytes = SLORA_RING_KB * 1024;  // ring + control block stay b
 // measured 2 % slower with it and keep kRingBytes.
 constexpr int kExpandRingBytes = SLORA_EXPAND_RING_KB * 1024;
 constexpr int kPipeCtasPerSm = 2;      // persistent CTAs per SM
-constexpr int kPendSlots = 4;           // stages that may be issued before the grid-dependency wait
-constexpr int kProducerWarps = 1;  // stage g is fed by producer warp g % kProducerWarps
+// Producer warps: the first resolves items and copies adapter rows, the second copies activations.
+constexpr int kProducerWarps = 2;
+constexpr int kRowsAhead = 3;  // a CTA's first stages: all their adapter rows are the first producer's
 constexpr int kConsumerWarps = 8;
 constexpr int kPipeThreads = 32 * (kProducerWarps + kConsumerWarps);
 constexpr int kMaxStageBytes = SLORA_STAGE_KB * 1024;  // a shrink item is cut into K-chunks no larger than this
 constexpr int kPipeChunk = 16384;          // flat B elements per expand item (32 KB)
-constexpr int kMaxPieces = 16;  // B copies per expand stage (lanes 0..15); y copies use lanes 16..23, delta 24..31
-constexpr int kSpanRows = 6;    // pool rows a B chunk may touch
-constexpr int kWideRows = 8;    // adapter rows of a shrink item of a tile with at most kWideTokens tokens (EXACT only)
-constexpr int kWideTokens = 4;
+constexpr int kSpanRows = 6;    // pool rows a B chunk may touch: one copy each (lanes 0..5); y copies use lanes
+                                // 16..23, delta rows 24..31
+constexpr int kItemRows = 16;   // widest shrink item: adapter rows (ShrinkArgs::rows_per_cta picks 4, 8 or 16)
+constexpr int kActLane = 16;    // lanes kActLane.. carry a stage's activation copies
 constexpr int kCompactTiles = 640;  // tiles whose item counts fit the control block (two CTAs per SM leave little room)
 
 constexpr int FLAG_FIRST = 1, FLAG_LAST = 2, FLAG_END = 4;
@@ -86,18 +98,12 @@ struct PipeCtl {
   uint64_t full[kSlots];
   uint64_t empty[kSlots];
   int meta[kSlots][16];
-  // one private copy per producer warp of everything below
-  struct Prod {
-    uint32_t off[kSlots];  // byte offset of each stage in the ring
-    // activation copies of the stages issued before the grid-dependency wait (one entry per lane)
-    uint64_t pend_src[kPendSlots][32];
-    uint32_t pend_dst[kPendSlots][32];
-    uint32_t pend_bytes[kPendSlots][32];
-    // the 32 items a batch resolves, one per lane, parked here so that the lanes that carry the copies read what
-    // they need instead of receiving it through shuffles
-    int64_t d_l[32][kWideRows];
-    int d_i[32][16];
-  } prod[kProducerWarps];
+  uint32_t off[kProducerWarps][kSlots];  // byte offset of each stage in the ring (a copy per producer warp)
+  // the 32 items a batch resolves, one per lane of the first producer warp, parked here for the lanes that carry the
+  // copies: pool rows and the item's description
+  int32_t d_l[32][kItemRows];
+  int d_i[32][16];
+  uint32_t valid_mask;
   // planned batches of mixed ranks: items up to and including each tile (see build_item_map)
   uint16_t item_end[kCompactTiles];
   int tp_gave_up;  // in-band signalling: a wait for another rank's values ran out; nobody in this CTA waits again
@@ -105,8 +111,10 @@ struct PipeCtl {
 
 // Shrink only: per-item partial sums of the consumer warps and the arrival counter that elects the last warp.  (Kept
 // out of PipeCtl so that the expand, which has no use for it, can give those 8 KB to its ring.)
+// Rows of a C fragment: half h holds rows 8h + lane / 4, tokens 2 (lane % 4) and the next; four, eight or sixteen rows
+// are a half fragment (the lanes below 16), one or two.  8 KB hold the items that shrink_slots() lets be in flight.
 struct ShrinkRed {
-  float sum[kSlots][kConsumerWarps][32];
+  float2 sum[4 * kConsumerWarps * 32];
   int cnt[kSlots];
 };
 
@@ -117,9 +125,9 @@ struct Ring {
   uint32_t tail = 0;  // oldest stage not yet known to be released
   uint32_t head = 0;  // next free byte
   bool pre = true;    // still before the grid-dependency wait
-  int npend = 0;      // stages with stashed activation copies
   bool dead = false;  // a bounded wait ran out
   uint32_t cap = kRingBytes;  // bytes of the ring
+  uint32_t slots = kSlots;    // stages in flight at most
   const TpLink* tp = nullptr;  // expand under tensor parallelism: flags to wait for before activations are read
   int32_t* status = nullptr;
   bool trigger_after_wait = false;  // shrink whose expand starts early: dependents may launch once this has waited
@@ -235,30 +243,22 @@ __device__ __forceinline__ void tp_inband_finish(const TpLink& tp, void* half_ba
   if (threadIdx.x == 0) *tp.counter = 0;
 }
 
-__device__ __forceinline__ void ring_flush(Ring& r, PipeCtl& c, int lane) {
+// The grid-dependency wait of a producer warp.  The one that copies activations does it before its first copy (and, under
+// tensor parallelism with flags, waits for the other ranks' there); the one that copies adapter rows, which no kernel
+// on the stream writes, only before it first waits for ring space.
+__device__ __forceinline__ void ring_enter(Ring& r, int lane) {
+  if (!r.pre) return;
+  r.pre = false;
   pdl_wait();
   if (r.trigger_after_wait) pdl_launch_dependents();
-  if (r.tp != nullptr && !r.tp->inband && !tp_link_wait(*r.tp, lane)) {
+  if (r.role != 0 && r.tp != nullptr && !r.tp->inband && !tp_link_wait(*r.tp, lane)) {
     // the copies still go out (the consumers' barriers expect them); the result is flagged as not to be trusted
     if (lane == 0) set_status(r.status, SLORA_STATUS_TIMEOUT);
   }
-  PipeCtl::Prod& pp = c.prod[r.role];
-  for (int i = 0; i < r.npend; ++i) {
-    const uint32_t slot = (r.g - r.npend + i) % kSlots;
-    if (pp.pend_bytes[i][lane] != 0) {
-      asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(
-                       pp.pend_dst[i][lane]),
-                   "l"(pp.pend_src[i][lane]), "r"(pp.pend_bytes[i][lane]), "r"(smem_u32(&c.full[slot]))
-                   : "memory");
-    }
-  }
-  r.npend = 0;
-  r.pre = false;
 }
 
 // Reserve `sz` bytes (a multiple of 128) and a descriptor for stage r.g; returns the byte offset, or 0xffffffff when
-// a wait ran out.  Before the grid-dependency wait no stage has been released yet, so running out of room there
-// ends the prologue (ring_flush) instead of waiting.
+// a wait ran out.
 __device__ __forceinline__ uint32_t ring_alloc(Ring& r, PipeCtl& c, uint32_t sz, int lane) {
   for (;;) {
     uint32_t cand = 0;
@@ -267,7 +267,7 @@ __device__ __forceinline__ uint32_t ring_alloc(Ring& r, PipeCtl& c, uint32_t sz,
       r.head = 0;
       ok = true;
     } else {
-      const uint32_t t = c.prod[r.role].off[r.tail % kSlots];
+      const uint32_t t = c.off[r.role][r.tail % kSlots];
       if (r.head > t) {
         if (r.head + sz <= r.cap) {
           cand = r.head;
@@ -281,11 +281,8 @@ __device__ __forceinline__ uint32_t ring_alloc(Ring& r, PipeCtl& c, uint32_t sz,
         ok = r.head + sz <= t && r.head != t;
       }
     }
-    if (ok && r.g - r.tail < kSlots && !(r.pre && r.npend == kPendSlots)) return cand;
-    if (r.pre) {
-      ring_flush(r, c, lane);
-      continue;
-    }
+    if (ok && r.g - r.tail < r.slots) return cand;
+    ring_enter(r, lane);
     if (!mbar_wait_timed(&c.empty[r.tail % kSlots], (r.tail / kSlots) & 1)) {
       r.dead = true;
       return 0xffffffffu;
@@ -294,37 +291,36 @@ __device__ __forceinline__ uint32_t ring_alloc(Ring& r, PipeCtl& c, uint32_t sz,
   }
 }
 
-// One bulk instruction for the whole stage: lane `lane` carries (dst, src, bytes) or bytes == 0.  Activation copies
-// (is_act) issued before the grid-dependency wait are stashed instead.
+// The copies of a stage: lane `lane` carries (dst, src, bytes) or bytes == 0.  A bulk copy's operands are uniform
+// registers, so a warp issues its lanes' copies one after the other (measured on B200: 52 cycles a copy with the SM to
+// itself, 75 to 140 beside working consumers), while two warps issue side by side: each producer warp works out the same
+// stages and calls this for its share of the lanes.  The stage's byte count is announced by one arrival (the first
+// warp's); copies of the other warp may complete before it.
 __device__ __forceinline__ void ring_issue(Ring& r, PipeCtl& c, uint32_t slot, uint32_t dst, const void* src,
-                                           uint32_t bytes, bool is_act, int lane) {
-  if (static_cast<int>(r.g % kProducerWarps) != r.role) bytes = 0;  // the other producer's stage
-  if (r.pre) {
-    PipeCtl::Prod& pp = c.prod[r.role];
-    pp.pend_bytes[r.npend][lane] = is_act ? bytes : 0;
-    pp.pend_dst[r.npend][lane] = dst;
-    pp.pend_src[r.npend][lane] = reinterpret_cast<uint64_t>(src);
-    if (is_act) bytes = 0;
-  }
+                                           uint32_t bytes) {
   if (bytes != 0) {
     asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(dst),
                  "l"(src), "r"(bytes), "r"(smem_u32(&c.full[slot]))
                  : "memory");
   }
-  if (r.pre) ++r.npend;
   ++r.g;
+}
+
+// The producer warps meet: before a batch of items is resolved (all of them are done with the previous one) and after.
+__device__ __forceinline__ void producers_sync() {
+  asm volatile("bar.sync 1, %0;" ::"n"(kProducerWarps * 32) : "memory");
 }
 
 // Finish: flush a prologue that never ended, then post the end marker.
 __device__ __forceinline__ void ring_finish(Ring& r, PipeCtl& c, int32_t* status, int lane) {
-  if (r.pre) ring_flush(r, c, lane);
+  ring_enter(r, lane);
   if (!r.dead) ring_alloc(r, c, 0, lane);
   if (r.dead) {
     if (lane == 0) set_status(status, SLORA_STATUS_TIMEOUT);
     return;
   }
   const uint32_t slot = r.g % kSlots;
-  if (lane == 0 && static_cast<int>(r.g % kProducerWarps) == r.role) {
+  if (lane == 0 && r.role == 0) {
     c.meta[slot][0] = FLAG_END;
     mbar_arrive(&c.full[slot]);
   }
@@ -406,7 +402,7 @@ __device__ __forceinline__ void fill_item_counts(const TileSrc& src, const Table
 // item_end become running counts (each lane sums a contiguous run, the warp scans the lane sums).
 template <typename F>
 __device__ __forceinline__ ItemMap build_item_map(const TileSrc& src, int padded_per_tile, PipeCtl& c, int lane,
-                                                  F items_of_rank) {
+                                                  int role, F items_of_rank) {
   ItemMap m;
   m.per_tile = padded_per_tile;
   if (src.mode != MODE_PLAN) {
@@ -437,12 +433,15 @@ __device__ __forceinline__ ItemMap build_item_map(const TileSrc& src, int padded
   }
   const int total = __shfl_sync(FULL_MASK, incl, 31);
   if (total > 0xffff) return m;  // too many items for 16-bit counts (same decision in every lane)
-  int run = incl - sum;
-  for (int i = lo; i < hi; ++i) {
-    run += c.item_end[i];
-    c.item_end[i] = static_cast<uint16_t>(run);
+  producers_sync();  // every producer warp has read the counts; one of them turns them into running counts
+  if (role == 0) {
+    int run = incl - sum;
+    for (int i = lo; i < hi; ++i) {
+      run += c.item_end[i];
+      c.item_end[i] = static_cast<uint16_t>(run);
+    }
   }
-  __syncwarp();
+  __syncwarp();  // (only the first producer warp looks items up)
   m.mode = 2;
   m.n_items = total;
   return m;
@@ -463,9 +462,15 @@ __device__ __forceinline__ int64_t padded_item_count(const TileSrc& src, int pad
 }
 
 // Item q -> its tile and its index among that tile's items.
-__device__ __forceinline__ void item_to_tile(const ItemMap& m, const PipeCtl& c, int64_t q, int& tile, int& local) {
+__device__ __forceinline__ void item_to_tile(const ItemMap& m, const FastDiv& padded, const PipeCtl& c, int64_t q,
+                                             int& tile, int& local) {
   if (m.mode != 2) {
-    tile = static_cast<int>(q / m.per_tile);
+    if (q < 0x7fffffff) {
+      const uint32_t q32 = static_cast<uint32_t>(q);
+      tile = m.mode == 0 ? padded.div(static_cast<int>(q32)) : static_cast<int>(q32 / static_cast<uint32_t>(m.per_tile));
+    } else {
+      tile = static_cast<int>(q / m.per_tile);
+    }
     local = static_cast<int>(q - static_cast<int64_t>(tile) * m.per_tile);
     return;
   }
@@ -487,19 +492,52 @@ __device__ __forceinline__ void item_to_tile(const ItemMap& m, const PipeCtl& c,
 // stage meta: [0] flags [1] nrows [2] n [3] j0 [4] projection [5] klen [6] ring offset, [8..15] token ids
 // stage bytes: nrows chunks of klen elements (adapter rows), then n chunks of klen elements (token rows)
 // ------------------------------------------------------------------------------------------------------------
-// Row blocks a tile of rr slot rows has per projection (blocks of kWideRows rows when `wide`, else kMaxRows; rows
-// beyond the delta buffers' width are not enumerated), and its items.
+// Row blocks a tile of rr slot rows has per projection (rows beyond the delta buffers' width are not enumerated).
 __device__ __forceinline__ int shrink_rows_of(const ShrinkArgs& a, int rr) {
-  return min(rr * a.rank_mult, a.max_rb * kMaxRows);
+  return min(rr * a.rank_mult, a.max_rb * a.rows_per_cta);
 }
-__device__ __forceinline__ int shrink_blocks_of(const ShrinkArgs& a, int rr, bool wide) {
-  const int per = wide ? kWideRows : kMaxRows;
-  return (shrink_rows_of(a, rr) + per - 1) / per;
+__device__ __forceinline__ int shrink_blocks_of(const ShrinkArgs& a, int rr) {
+  return (shrink_rows_of(a, rr) + a.rows_per_cta - 1) >> (31 - __clz(a.rows_per_cta));  // 4, 8 or 16
 }
-// With per-tile counts (ranks differ) a tile of few tokens takes its rows eight at a time: its token rows are then
-// staged once per eight adapter rows instead of once per four.
-__device__ __forceinline__ int shrink_items_of(const ShrinkArgs& a, int rr, int n) {
-  return a.nproj * shrink_blocks_of(a, rr, n <= kWideTokens);
+__device__ __forceinline__ int shrink_items_of(const ShrinkArgs& a, int rr) { return a.nproj * shrink_blocks_of(a, rr); }
+
+// Item `rem` of a tile's nb items per projection: which projection (the last one takes what is beyond: its row block
+// is then past the adapter's rows).
+__device__ __forceinline__ int proj_of(int rem, int nb, int nproj) {
+  return min((rem >= nb ? 1 : 0) + (rem >= 2 * nb ? 1 : 0), nproj - 1);
+}
+
+// Chunk j of a stage starts (j + 1) / 2 * kChunkPad bytes after j chunks' values: two rows that lie next to each other
+// start in different halves of the banks, so that the eight lanes that read 64 bytes of each do not collide.
+constexpr int kChunkPad = 64;
+__device__ __forceinline__ int chunk_at(int j, int bytes) { return j * bytes + ((j + 1) >> 1) * kChunkPad; }
+// K elements of a shrink stage of `chunks` rows and tokens, in pairs of units of kKUnit: what fits kMaxStageBytes, at
+// least one pair.
+constexpr int kKUnit = 512;
+constexpr int stage_pairs(int c) {
+  const int p = (kMaxStageBytes - 64 - (c + 1) / 2 * kChunkPad) / (c * kKUnit * 4);
+  return p < 1 ? 1 : (p > 255 ? 255 : p);
+}
+struct StagePairs {
+  uint64_t w[3];  // a byte per number of chunks (1..24)
+};
+constexpr StagePairs stage_pairs_table() {
+  StagePairs s = {{0, 0, 0}};
+  for (int c = 1; c <= 24; ++c) s.w[(c - 1) / 8] |= static_cast<uint64_t>(stage_pairs(c)) << (8 * ((c - 1) % 8));
+  return s;
+}
+constexpr uint64_t kPairs0 = stage_pairs_table().w[0], kPairs1 = stage_pairs_table().w[1],
+                   kPairs2 = stage_pairs_table().w[2];
+__device__ __forceinline__ int stage_k(int chunks) {
+  const int i = chunks - 1;
+  const uint64_t w = i < 8 ? kPairs0 : (i < 16 ? kPairs1 : kPairs2);
+  return static_cast<int>((w >> (8 * (i & 7))) & 255u) * (2 * kKUnit);
+}
+// Reduction buffers (items in flight) and stages in flight of a launch.  Stages in flight touch at most one item more
+// than the whole items among them: three stages of items of two or more are two items.
+__device__ __forceinline__ uint32_t shrink_buffers(int rows_per_item) { return rows_per_item > 8 ? 2 : (rows_per_item > 4 ? 4 : 8); }
+__device__ __forceinline__ uint32_t shrink_slots(int rows_per_item, int h_in) {
+  return rows_per_item > 8 ? (h_in > stage_k(kItemRows + 1) ? 3 : 2) : shrink_buffers(rows_per_item);
 }
 
 template <typename T, bool EXACT>
@@ -511,125 +549,154 @@ __device__ __forceinline__ void shrink_producer(const ShrinkArgs& a, unsigned ch
   const T* x = reinterpret_cast<const T*>(a.x);
   const int64_t G = gridDim.x;
   const uint32_t ring_base = smem_u32(ring_mem);
-  PipeCtl::Prod& pp = c.prod[role];
+  const int RB = a.rows_per_cta;
   Ring r;
   r.role = role;
+  r.cap = kShrinkRingBytes;
+  r.slots = shrink_slots(RB, h_in);
   r.trigger_after_wait = a.tp.enabled && a.tp.inband >= 2;
-  constexpr int RMAX = EXACT ? kWideRows : kMaxRows;  // rows of the widest item = lane of the first token row
-  const ItemMap map = EXACT ? build_item_map(a.src, a.nproj * a.max_rb, c, lane,
-                                             [&](int rr, int) { return a.nproj * shrink_blocks_of(a, rr, false); })
+  const ItemMap map = EXACT ? build_item_map(a.src, a.nproj * a.max_rb, c, lane, role,
+                                             [&](int rr, int) { return shrink_items_of(a, rr); })
                             : padded_item_map(a.src, a.nproj * a.max_rb);
   const int mode = EXACT ? map.mode : 0;
   int64_t n_items = map.n_items;
-  const int rows_per_pool_row = static_cast<int>(S / h_in);  // the pipelined shrink is given S % h_in == 0
+  const int rpp = static_cast<int>(a.rows_per_row.d);  // A rows per pool row (a whole number here)
 
-  for (int64_t batch0 = blockIdx.x; batch0 < n_items && !r.dead; batch0 += 32 * G) {
-    // ---- 32 items resolved in parallel, one per lane; d_i[lane] = {valid, n, nrows, j0, p, -, -, -, tok[8]} ----
-    const int64_t item = batch0 + lane * G;
-    int valid = 0;
-    if (item < n_items) {
-      int tile, rem;
-      item_to_tile(map, c, item, tile, rem);
-      // projection and row block: known before the tile record arrives unless ranks are mixed
-      int nb = mode == 0 ? a.max_rb : shrink_blocks_of(a, map.uniform, false);
-      // resolved tiles: where projection and row block follow from the item index alone, the pool rows of the
-      // item are fetched now, together with the header and the record that will say whether they count
-      int spec_row[kMaxRows];
-      bool spec = false;
-      if (a.src.mode == MODE_PLAN && a.src.xoff > 0 && mode != 2) {
-        const int p_s = min(rem / nb, a.nproj - 1), rb_s = rem - (rem / nb) * nb;
-        const int32_t* xt = a.src.plan + a.src.xoff + static_cast<int64_t>(tile) * (kXtHead + 4 * a.src.xrcap);
-        const int qk_s = pick3(a.qkvo, p_s);
+  // (a producer warp whose wait ran out goes on meeting the other one)
+  for (int64_t batch0 = blockIdx.x; batch0 < n_items; batch0 += 32 * G) {
+    producers_sync();
+    // ---- 32 items resolved in parallel, one per lane of the first producer warp:
+    //      d_i[lane] = {-, n, nrows, j0, p, slot rows, -, -, tok[8]}, d_l[lane] = pool row of each A row ----
+    if (role == 0) {
+      const int64_t item = batch0 + lane * G;
+      int valid = 0;
+      if (item < n_items) {
+        int tile, rem;
+        item_to_tile(map, a.per_tile, c, item, tile, rem);
+        // projection and row block: known before the tile record arrives unless ranks are mixed
+        int nb = mode == 0 ? a.max_rb : shrink_blocks_of(a, map.uniform);
+        // resolved tiles: where projection and row block follow from the item index alone, the pool rows of the
+        // item are fetched now, together with the header and the record that will say whether they count
+        int4 rows4[kItemRows / 4];
+        const bool entry = a.src.mode == MODE_PLAN && a.src.xoff > 0 && rpp == 1;
+        auto fetch_rows = [&](int qk, int j0) {
+          const int32_t* xt = a.src.plan + a.src.xoff + static_cast<int64_t>(tile) * (kXtHead + 4 * a.src.xrcap) + kXtHead +
+                              qk * a.src.xrcap;
 #pragma unroll
-        for (int j = 0; j < kMaxRows; ++j) {
-          const int pr = (rb_s * kMaxRows + j) / rows_per_pool_row;
-          spec_row[j] = xt[kXtHead + qk_s * a.src.xrcap + min(pr, a.src.xrcap - 1)];
+          for (int v = 0; v < kItemRows / 4; ++v) {
+            rows4[v] = make_int4(-1, -1, -1, -1);
+            if (4 * v < RB && j0 + 4 * v < a.src.xrcap) rows4[v] = *reinterpret_cast<const int4*>(xt + j0 + 4 * v);
+          }
+        };
+        if (entry && mode != 2) {
+          const int p_s = proj_of(rem, nb, a.nproj);
+          fetch_rows(pick3(a.qkvo, p_s), (rem - p_s * nb) * RB);
         }
-        spec = true;
-      }
-      TileInfo t;
-      if (lookup_tile(a.src, a.tb, tile, t, a.status)) {
-        const bool wide = mode == 2 && t.n <= kWideTokens;
-        if (mode == 2) nb = shrink_blocks_of(a, t.r, wide);
-        const int per = wide ? kWideRows : kMaxRows;
-        const int p = rem / nb, rb = rem - p * nb;
-        const int j0 = rb * per;
-        const int rows_total = shrink_rows_of(a, t.r);  // A rows of the projection (rows may be shorter than a pool row)
-        if (p < a.nproj && j0 < rows_total) {
-          const int nrows = min(per, rows_total - j0);
-          const int qk = pick3(a.qkvo, p);
-          bool ok = true;
+        TileInfo t;
+        if (lookup_tile(a.src, a.tb, tile, t, a.status)) {
+          if (mode == 2) nb = shrink_blocks_of(a, t.r);
+          const int p = proj_of(rem, nb, a.nproj), j0 = (rem - p * nb) * RB;
+          const int rows_total = shrink_rows_of(a, t.r);  // A rows of the projection (rows may be shorter than a pool row)
+          if (j0 < rows_total) {
+            const int nrows = min(RB, rows_total - j0);
+            const int qk = pick3(a.qkvo, p);
+            bool ok = true;
+            if (entry && t.xok) {
+              if (j0 + nrows > t.r) ok = false;
+              if (mode == 2) fetch_rows(qk, j0);
 #pragma unroll
-          for (int j = 0; j < RMAX; ++j) {
-            if (j < nrows) {
-              const int64_t f = static_cast<int64_t>(j0 + j) * h_in;
-              const int64_t pr = f / S, col = f - pr * S;
-              int64_t e = -1;
-              if (pr < t.r) e = (spec && t.xok && j < kMaxRows) ? spec_row[j < kMaxRows ? j : 0] : tile_loc(t, a.tb, qk, pr);
-              if (e < 0 || e >= a.tb.pool_rows) ok = false;
-              pp.d_l[lane][j] = e * S + col;
+              for (int v = 0; v < kItemRows / 4; ++v) {
+                if (4 * v < nrows) {
+                  const int4 e = rows4[v];
+                  auto bad = [&](int row, int j) { return j < nrows && (row < 0 || row >= a.tb.pool_rows); };
+                  if (bad(e.x, 4 * v) || bad(e.y, 4 * v + 1) || bad(e.z, 4 * v + 2) || bad(e.w, 4 * v + 3)) ok = false;
+                  *reinterpret_cast<int4*>(&c.d_l[lane][4 * v]) = e;
+                }
+              }
+            } else {
+              for (int v = 0; v < nrows; v += 4) {
+                int64_t e[4];  // four loads in flight
+#pragma unroll
+                for (int j = 0; j < 4; ++j) {
+                  const int pr = a.rows_per_row.div(min(j0 + v + j, rows_total - 1));
+                  e[j] = pr < t.r ? tile_loc(t, a.tb, qk, pr) : -1;
+                }
+#pragma unroll
+                for (int j = 0; j < 4; ++j) {
+                  if (e[j] < 0 || e[j] >= a.tb.pool_rows) ok = false;
+                  c.d_l[lane][v + j] = static_cast<int32_t>(e[j]);  // (pool_rows < 2^31 here)
+                }
+              }
+            }
+            if (ok) {
+              int tok[kTileTokens];
+#pragma unroll
+              for (int i = 0; i < kTileTokens; ++i) tok[i] = i < t.n ? tile_token(t, i) : 0;
+              int4* di = reinterpret_cast<int4*>(c.d_i[lane]);
+              di[0] = make_int4(0, t.n, nrows, j0);
+              di[1] = make_int4(p, t.r, 0, 0);
+              di[2] = make_int4(tok[0], tok[1], tok[2], tok[3]);
+              di[3] = make_int4(tok[4], tok[5], tok[6], tok[7]);
+              valid = 1;
+            } else {
+              set_status(a.status, SLORA_STATUS_BAD_TABLE);
             }
           }
-          if (ok) {
-#pragma unroll
-            for (int i = 0; i < kTileTokens; ++i) pp.d_i[lane][8 + i] = i < t.n ? tile_token(t, i) : 0;
-            pp.d_i[lane][1] = t.n;
-            pp.d_i[lane][2] = nrows;
-            pp.d_i[lane][3] = j0;
-            pp.d_i[lane][4] = p;
-            pp.d_i[lane][5] = t.r;
-            valid = 1;
-          } else {
-            set_status(a.status, SLORA_STATUS_BAD_TABLE);
-          }
         }
       }
+      const uint32_t mask = __ballot_sync(FULL_MASK, valid != 0);
+      if (lane == 0) c.valid_mask = mask;
     }
-    const uint32_t valid_mask = __ballot_sync(FULL_MASK, valid != 0);
-    __syncwarp();
+    producers_sync();
+    const uint32_t valid_mask = c.valid_mask;
 
-    // ---- feed the ring, item by item (lane j < RMAX carries adapter row j, lane RMAX + i carries token i) ----
+    // ---- feed the ring, item by item (lane j < 16 carries adapter row j, lane 16 + i carries token i) ----
     for (uint32_t left = valid_mask; left != 0 && !r.dead; left &= left - 1) {
       const int k = __ffs(left) - 1;
-      const int* di = pp.d_i[k];
-      const int n = di[1], nrows = di[2];
+      const int* di = c.d_i[k];
+      const int4 d0 = *reinterpret_cast<const int4*>(di);
+      const int n = d0.y, nrows = d0.z, m_j0 = d0.w, m_p = di[4], m_rows = di[5];
       const bool is_w = lane < nrows;
-      const bool is_x = lane >= RMAX && lane < RMAX + n;
-      const int mytok = (lane >= RMAX && lane < RMAX + kTileTokens) ? di[8 + lane - RMAX] : 0;
-      const T* src0 = is_w ? w + pp.d_l[k][lane & (RMAX - 1)] : x + static_cast<int64_t>(mytok) * a.x_stride;
-      const int myslot = is_w ? lane : nrows + (lane - RMAX);  // position of this lane's chunk in the stage
-      const int m_j0 = di[3], m_p = di[4], m_rows = di[5];
-      // cut the item into K-chunks that are multiples of 2048 elements (so the element -> consumer lane mapping, and
-      // with it the summation order, does not depend on how many tokens share the tile) and, where that allows,
-      // no larger than kMaxStageBytes
-      const int fit = kMaxStageBytes / ((nrows + n) * static_cast<int>(sizeof(T))) / 2048 * 2048;
-      const int kc_elems = fit < 2048 ? 2048 : fit;
+      const bool is_x = lane >= kActLane && lane < kActLane + n;
+      const int mytok = lane >= kActLane ? di[8 + (lane & 7)] : 0;
+      const T* src0;
+      if (lane < kActLane) {
+        const int row = m_j0 + lane;
+        const int pr = a.rows_per_row.div(row);
+        src0 = w + c.d_l[k][lane] * S + static_cast<int64_t>(row - pr * rpp) * h_in;
+      } else {
+        src0 = x + static_cast<int64_t>(mytok) * a.x_stride;
+      }
+      const int myslot = is_w ? lane : nrows + (lane - kActLane);  // position of this lane's chunk in the stage
+      // the item goes through the ring in K-chunks of whole units of kKUnit elements (so the element -> consumer lane
+      // mapping, and with it the summation order, does not depend on how many rows or tokens share the stage)
+      const int kc_elems = stage_k(nrows + n);
       for (int k0 = 0; k0 < h_in; k0 += kc_elems) {
         const int klen = min(kc_elems, h_in - k0);
         const uint32_t bytes = static_cast<uint32_t>(klen) * sizeof(T);
-        const uint32_t sz = round128(static_cast<uint32_t>(nrows + n) * bytes);
+        const uint32_t sz = round128(chunk_at(nrows + n, bytes));
         const uint32_t off = ring_alloc(r, c, sz, lane);
         if (r.dead) break;
         const uint32_t slot = r.g % kSlots;
-        const bool mine = static_cast<int>(r.g % kProducerWarps) == role;
         r.head = off + sz;
-        if (lane == 0) pp.off[slot] = off;
-        if (!mine) {
-          __syncwarp();
-          ring_issue(r, c, slot, 0, nullptr, 0u, false, lane);
-          continue;
+        if (lane == 0) c.off[role][slot] = off;
+        if (role == 0) {
+          if (lane == 0) {  // the stage record in two 16-byte stores; [7] = slot rows of the adapter
+            int4* mrec = reinterpret_cast<int4*>(c.meta[slot]);
+            mrec[0] = make_int4((k0 == 0 ? FLAG_FIRST : 0) | (k0 + klen >= h_in ? FLAG_LAST : 0), nrows, n, m_j0);
+            mrec[1] = make_int4(m_p, klen, static_cast<int>(off), m_rows);
+          } else if (lane >= kActLane && lane < kActLane + kTileTokens) {
+            c.meta[slot][8 + lane - kActLane] = mytok;
+          }
+          __syncwarp();  // the arrive below publishes every lane's part of the stage record
+          if (lane == 0) mbar_expect_tx(&c.full[slot], static_cast<uint32_t>(nrows + n) * bytes);
         }
-        if (lane == 0) {  // the stage record in two 16-byte stores; [7] = slot rows of the adapter
-          int4* mrec = reinterpret_cast<int4*>(c.meta[slot]);
-          mrec[0] = make_int4((k0 == 0 ? FLAG_FIRST : 0) | (k0 + klen >= h_in ? FLAG_LAST : 0), nrows, n, m_j0);
-          mrec[1] = make_int4(m_p, klen, static_cast<int>(off), m_rows);
-        } else if (lane >= RMAX && lane < RMAX + kTileTokens) {
-          c.meta[slot][8 + lane - RMAX] = mytok;
-        }
-        __syncwarp();  // the arrive below publishes every lane's part of the stage record
-        if (lane == 0) mbar_expect_tx(&c.full[slot], static_cast<uint32_t>(nrows + n) * bytes);
-        ring_issue(r, c, slot, ring_base + off + static_cast<uint32_t>(myslot) * bytes, src0 + k0,
-                   (is_w || is_x) ? bytes : 0u, is_x, lane);
+        // after a CTA's first stages the second producer takes some of the rows as well: half of all copies each
+        if (role != 0) ring_enter(r, lane);
+        const bool mine = role == 0 ? is_w && (r.g < kRowsAhead || lane < (nrows + n + 1) / 2)
+                                    : is_x || (is_w && r.g >= kRowsAhead && lane >= (nrows + n + 1) / 2);
+        ring_issue(r, c, slot, ring_base + off + chunk_at(myslot, bytes), src0 + k0,
+                   mine ? bytes : 0u);
       }
     }
     __syncwarp();
@@ -638,87 +705,106 @@ __device__ __forceinline__ void shrink_producer(const ShrinkArgs& a, unsigned ch
   ring_finish(r, c, a.status, lane);
 }
 
-// Warp-level part of the per-item reduction: V = 4 * NT partial sums per lane (row-major [row][token]) are summed
-// across the warp and handed to the cross-warp buffer; lane l ends up with the total of index l >> (5 - log2 V).
-template <int NT>
-__device__ __forceinline__ void shrink_warp_reduce(const float (&acc)[kMaxRows][kTileTokens], float* red_row, int lane) {
-  constexpr int V = kMaxRows * NT;
-  float v[V];
-#pragma unroll
-  for (int j = 0; j < kMaxRows; ++j) {
-#pragma unroll
-    for (int i = 0; i < NT; ++i) v[j * NT + i] = acc[j][i];
-  }
-  const float tot = warp_reduce_scatter<V>(v, lane);
-  constexpr int SH = V == 32 ? 0 : (V == 16 ? 1 : (V == 8 ? 2 : 3));
-  if ((lane & ((1 << SH) - 1)) == 0) red_row[lane >> SH] = tot;
+// Sums of one warp over its slices of an item.  K goes by units of kKUnit elements; warp cw owns [cw * 64, +64) of each, two
+// fragments of 32.  Four sums are kept apart (unit odd or even, first or second fragment), four short chains of mma
+// instead of one long one, and added in one order at the end.  The two of a unit's fragments may share one instruction:
+// where rows and tokens leave half of it empty (SPLIT), the second fragment's rows and tokens take those places.
+struct ShrinkAcc {
+  float d[2][2][4];  // [unit parity][fragment; 0 alone when they share][C fragment]
+};
+enum ShrinkForm {
+  FORM_FULL,   // rows 0..7 and 8..15, tokens 0..7
+  FORM_WIDE,   // rows 0..7, tokens 0..7
+  FORM_ROWS8,  // rows 0..7, tokens 0..3: the second fragment in rows 8..15 and columns 4..7
+  FORM_ROWS4   // rows 0..3, tokens 0..3: the second fragment in rows 4..7 and columns 4..7
+};
+__device__ __forceinline__ int shrink_form(int rows_per_item, int nrows, int n) {
+  if (rows_per_item > 8) return FORM_FULL;
+  if (n > 4) return FORM_WIDE;
+  return nrows > 4 ? FORM_ROWS8 : FORM_ROWS4;
 }
 
-// Multiply-accumulate part of a shrink stage for a tile of at most NT tokens, free of data-dependent branches (each
-// branch costs the lone warp of a scheduler ~10-20 cycles of resolve latency): rows and tokens beyond the real counts
-// are clamped to the last real one, so their accumulators hold duplicates that are never written out.
-template <typename T, int NT>
-__device__ __forceinline__ void shrink_accumulate(float (&acc)[kMaxRows][kTileTokens], const T* st, int nrows, int n,
-                                                  int klen, int cw, int lane) {
-  const T* xs = st + nrows * klen;
-  const T* wrow[kMaxRows];
-#pragma unroll
-  for (int j = 0; j < kMaxRows; ++j) wrow[j] = st + min(j, nrows - 1) * klen;
-  const T* xrow[NT];
-#pragma unroll
-  for (int i = 0; i < NT; ++i) xrow[i] = xs + min(i, n - 1) * klen;
+// Lane (g, t) reads 16-byte vector t of the 64 bytes of a row or token; rows and tokens beyond the real counts, and what
+// lies beyond the rows' end (rows end anywhere on a multiple of eight elements), are zero.  A stage starts at an even
+// unit.  The loads of a round are issued before its first mma: the warp has nothing else to hide their latency with.
+template <typename T, int FORM>
+__device__ __forceinline__ void shrink_accumulate(ShrinkAcc& acc, const unsigned char* st, int nrows, int n, int klen,
+                                                  int cw, int lane) {
+  constexpr bool SPLIT = FORM == FORM_ROWS8 || FORM == FORM_ROWS4;
+  constexpr int UNITS = FORM == FORM_ROWS4 ? 4 : 2;  // of a round
+  constexpr int NA = FORM == FORM_ROWS4 ? 1 : 2, NB = FORM == FORM_FULL ? 2 : 0, NX = SPLIT ? 1 : 2;
+  const int g = lane >> 2, t = lane & 3;
+  const int bytes = klen * static_cast<int>(sizeof(T));
+  const uint4 zero = make_uint4(0u, 0u, 0u, 0u);
+  const int row = FORM == FORM_ROWS4 ? (g & 3) : g, tok = SPLIT ? (g & 3) : g;
+  const int ka = cw * (kKUnit / kConsumerWarps) + 8 * t + (FORM == FORM_ROWS4 ? 32 * (g >> 2) : 0);
+  const int kx = cw * (kKUnit / kConsumerWarps) + 8 * t + (SPLIT ? 32 * (g >> 2) : 0);
+  // the first element a lane may not read any more (0: none of them)
+  const int end_a = row < nrows ? klen - ka : 0, end_b = FORM == FORM_FULL && g + 8 < nrows ? klen - ka : 0,
+            end_x = tok < n ? klen - kx : 0;
+  const unsigned char* pa = st + chunk_at(row, bytes) + ka * 2;
+  const unsigned char* pb = st + chunk_at(g + 8, bytes) + ka * 2;
+  const unsigned char* px = st + chunk_at(nrows + tok, bytes) + kx * 2;
 #pragma unroll 1
-  for (int k = cw * 256 + lane * 8; k < klen; k += kConsumerWarps * 256) {
-    uint4 wv[kMaxRows];
+  for (int k0 = 0; k0 < klen; k0 += UNITS * kKUnit) {
+    uint4 va[UNITS][NA], vb[UNITS][NB ? NB : 1], vx[UNITS][NX];
 #pragma unroll
-    for (int j = 0; j < kMaxRows; ++j) wv[j] = *reinterpret_cast<const uint4*>(wrow[j] + k);
+    for (int u = 0; u < UNITS; ++u) {
+      const int k = u * kKUnit;
 #pragma unroll
-    for (int i = 0; i < NT; ++i) {
-      const uint4 xv = *reinterpret_cast<const uint4*>(xrow[i] + k);
+      for (int h = 0; h < NA; ++h) va[u][h] = k0 + k + 32 * h < end_a ? *reinterpret_cast<const uint4*>(pa + 2 * (k + 32 * h)) : zero;
 #pragma unroll
-      for (int j = 0; j < kMaxRows; ++j) dot8<T>(acc[j][i], wv[j], xv);
+      for (int h = 0; h < NB; ++h) vb[u][h] = k0 + k + 32 * h < end_b ? *reinterpret_cast<const uint4*>(pb + 2 * (k + 32 * h)) : zero;
+#pragma unroll
+      for (int h = 0; h < NX; ++h) vx[u][h] = k0 + k + 32 * h < end_x ? *reinterpret_cast<const uint4*>(px + 2 * (k + 32 * h)) : zero;
+    }
+    pa += 2 * UNITS * kKUnit, pb += 2 * UNITS * kKUnit, px += 2 * UNITS * kKUnit;
+#pragma unroll
+    for (int u = 0; u < UNITS; ++u) {
+      float(&first)[4] = acc.d[u & 1][0];
+      float(&second)[4] = acc.d[u & 1][1];
+      const uint4 a0 = va[u][0], x0 = vx[u][0];
+      if (FORM == FORM_ROWS4) {
+        mma_k16<T>(first, a0.x, 0u, a0.y, 0u, x0.x, x0.y);
+        mma_k16<T>(first, a0.z, 0u, a0.w, 0u, x0.z, x0.w);
+      } else if (FORM == FORM_ROWS8) {
+        const uint4 a1 = va[u][NA - 1];
+        mma_k16<T>(first, a0.x, a1.x, a0.y, a1.y, x0.x, x0.y);
+        mma_k16<T>(first, a0.z, a1.z, a0.w, a1.w, x0.z, x0.w);
+      } else {
+        const uint4 a1 = va[u][NA - 1], x1 = vx[u][NX - 1];
+        const uint4 b0 = NB ? vb[u][0] : zero, b1 = NB ? vb[u][NB ? NB - 1 : 0] : zero;
+        mma_k16<T>(first, a0.x, b0.x, a0.y, b0.y, x0.x, x0.y);
+        mma_k16<T>(first, a0.z, b0.z, a0.w, b0.w, x0.z, x0.w);
+        mma_k16<T>(second, a1.x, b1.x, a1.y, b1.y, x1.x, x1.y);
+        mma_k16<T>(second, a1.z, b1.z, a1.w, b1.w, x1.z, x1.w);
+      }
     }
   }
 }
-
-// The same two steps for an item of kWideRows rows and at most kWideTokens tokens (NT in 1, 2, 4): the 32
-// accumulators are the same registers, indexed [row * NT + token].
-#define SLORA_ACC(idx) acc[(idx) >> 3][(idx) & 7]
-template <typename T, int NT>
-__device__ __forceinline__ void shrink_accumulate_wide(float (&acc)[kMaxRows][kTileTokens], const T* st, int nrows,
-                                                       int n, int klen, int cw, int lane) {
-  const T* xs = st + nrows * klen;
-#pragma unroll 1
-  for (int k = cw * 256 + lane * 8; k < klen; k += kConsumerWarps * 256) {
-    uint4 xv[NT];
+// The warp's partial sums in C-fragment order: [0], [1] row g columns 2t, 2t + 1; [2], [3] row g + 8.
+template <int FORM>
+__device__ __forceinline__ void shrink_partials(const ShrinkAcc& acc, float (&out)[4]) {
+  float first[4], second[4];
 #pragma unroll
-    for (int i = 0; i < NT; ++i) xv[i] = *reinterpret_cast<const uint4*>(xs + min(i, n - 1) * klen + k);
-#pragma unroll
-    for (int j = 0; j < kWideRows; ++j) {
-      const uint4 wv = *reinterpret_cast<const uint4*>(st + min(j, nrows - 1) * klen + k);
-#pragma unroll
-      for (int i = 0; i < NT; ++i) dot8<T>(SLORA_ACC(j * NT + i), wv, xv[i]);
-    }
+  for (int i = 0; i < 4; ++i) {
+    first[i] = acc.d[0][0][i] + acc.d[1][0][i];
+    second[i] = acc.d[0][1][i] + acc.d[1][1][i];
   }
-}
-template <int NT>
-__device__ __forceinline__ void shrink_warp_reduce_wide(const float (&acc)[kMaxRows][kTileTokens], float* red_row,
-                                                        int lane) {
-  constexpr int V = kWideRows * NT;
-  float v[V];
+  if (FORM == FORM_ROWS4) {  // the second fragment's sums sit four rows and four columns on: eighteen lanes
 #pragma unroll
-  for (int q = 0; q < V; ++q) v[q] = SLORA_ACC(q);
-  const float tot = warp_reduce_scatter<V>(v, lane);
-  constexpr int SH = V == 32 ? 0 : (V == 16 ? 1 : 2);
-  if ((lane & ((1 << SH) - 1)) == 0) red_row[lane >> SH] = tot;
+    for (int i = 0; i < 2; ++i) second[i] = __shfl_down_sync(FULL_MASK, first[i], 18);
+  } else if (FORM == FORM_ROWS8) {
+#pragma unroll
+    for (int i = 0; i < 2; ++i) second[i] = __shfl_down_sync(FULL_MASK, first[2 + i], 2);
+  }
+#pragma unroll
+  for (int i = 0; i < 4; ++i) out[i] = first[i] + second[i];
 }
-#undef SLORA_ACC
 
-// Consumer warp cw owns the K-slice [cw*256, +256) of every chunk: one 16-byte vector per lane per row / token, so a
-// stage is straight-line code with 4 * n independent FMA chains.  At the item's last chunk the warps' partial sums
-// meet in shared memory; the warp that arrives last (an atomic counter, no waiting) adds them in a fixed order and
-// writes delta.  A reduction buffer is reused only kSlots items later, which the ring guarantees to be after the
-// last warp released the stage it was summing in.
+// At the item's last chunk the warps' partial sums meet in shared memory; the warp that arrives last (an atomic counter,
+// no waiting) adds them in a fixed order and writes delta.  A reduction buffer is reused only as many items later as the
+// ring may hold stages, which is after the last warp released the stage it was summing in.
 template <typename T, bool EXACT>
 __device__ __forceinline__ void shrink_consumer(const ShrinkArgs& a, const unsigned char* ring_mem, PipeCtl& c,
                                                 ShrinkRed& red, int lane, int cw) {
@@ -744,12 +830,10 @@ __device__ __forceinline__ void shrink_consumer(const ShrinkArgs& a, const unsig
     __syncwarp();
   }
   if (a.tp.enabled && a.tp.inband >= 2) pdl_launch_dependents();
-  float acc[kMaxRows][kTileTokens];
-#pragma unroll
-  for (int j = 0; j < kMaxRows; ++j) {
-#pragma unroll
-    for (int i = 0; i < kTileTokens; ++i) acc[j][i] = 0.f;
-  }
+  const bool tall = a.rows_per_cta > 8;
+  const uint32_t buffers = shrink_buffers(a.rows_per_cta);
+  const int lanes = a.rows_per_cta > 4 ? 32 : 16;  // that hold rows of the item
+  ShrinkAcc acc = {};
   uint32_t item_seq = 0;
   for (uint32_t g = 0;; ++g) {
     const uint32_t slot = g % kSlots;
@@ -758,64 +842,33 @@ __device__ __forceinline__ void shrink_consumer(const ShrinkArgs& a, const unsig
       return;
     }
     const int* m = c.meta[slot];
-    const int flags = m[0];
+    const int4 m0 = *reinterpret_cast<const int4*>(m), m1 = *reinterpret_cast<const int4*>(m + 4);
+    const int flags = m0.x;
     if (flags & FLAG_END) return;
-    const int nrows = m[1], n = m[2], klen = m[5];
-    if (flags & FLAG_FIRST) {
-#pragma unroll
-      for (int j = 0; j < kMaxRows; ++j) {
-#pragma unroll
-        for (int i = 0; i < kTileTokens; ++i) acc[j][i] = 0.f;
-      }
-    }
-    const T* st = reinterpret_cast<const T*>(ring_mem + m[6]);
-    const bool wide = EXACT && nrows > kMaxRows;  // an item of up to kWideRows rows (the tile has <= kWideTokens tokens)
-    if (wide) {
-      if (n <= 1) {
-        shrink_accumulate_wide<T, 1>(acc, st, nrows, n, klen, cw, lane);
-      } else if (n <= 2) {
-        shrink_accumulate_wide<T, 2>(acc, st, nrows, n, klen, cw, lane);
-      } else {
-        shrink_accumulate_wide<T, 4>(acc, st, nrows, n, klen, cw, lane);
-      }
-    } else if (n <= 1) {
-      shrink_accumulate<T, 1>(acc, st, nrows, n, klen, cw, lane);
-    } else if (n <= 2) {
-      shrink_accumulate<T, 2>(acc, st, nrows, n, klen, cw, lane);
-    } else if (n <= 4) {
-      shrink_accumulate<T, 4>(acc, st, nrows, n, klen, cw, lane);
-    } else {
-      shrink_accumulate<T, 8>(acc, st, nrows, n, klen, cw, lane);
+    const int nrows = m0.y, n = m0.z, klen = m1.y;
+    if (flags & FLAG_FIRST) acc = ShrinkAcc{};
+    const unsigned char* st = ring_mem + m1.z;
+    const int form = shrink_form(a.rows_per_cta, nrows, n);
+    switch (form) {
+      case FORM_FULL: shrink_accumulate<T, FORM_FULL>(acc, st, nrows, n, klen, cw, lane); break;
+      case FORM_WIDE: shrink_accumulate<T, FORM_WIDE>(acc, st, nrows, n, klen, cw, lane); break;
+      case FORM_ROWS8: shrink_accumulate<T, FORM_ROWS8>(acc, st, nrows, n, klen, cw, lane); break;
+      default: shrink_accumulate<T, FORM_ROWS4>(acc, st, nrows, n, klen, cw, lane); break;
     }
     if (flags & FLAG_LAST) {
-      const uint32_t buf = item_seq % kSlots;
+      const uint32_t buf = item_seq % buffers;
       ++item_seq;
-      float* red_row = red.sum[buf][cw];
-      int nt;  // tokens rounded up to a power of two
-      if (wide) {
-        if (n <= 1) {
-          shrink_warp_reduce_wide<1>(acc, red_row, lane);
-          nt = 1;
-        } else if (n <= 2) {
-          shrink_warp_reduce_wide<2>(acc, red_row, lane);
-          nt = 2;
-        } else {
-          shrink_warp_reduce_wide<4>(acc, red_row, lane);
-          nt = 4;
-        }
-      } else if (n <= 1) {
-        shrink_warp_reduce<1>(acc, red_row, lane);
-        nt = 1;
-      } else if (n <= 2) {
-        shrink_warp_reduce<2>(acc, red_row, lane);
-        nt = 2;
-      } else if (n <= 4) {
-        shrink_warp_reduce<4>(acc, red_row, lane);
-        nt = 4;
-      } else {
-        shrink_warp_reduce<8>(acc, red_row, lane);
-        nt = 8;
+      // buffer of this item: eight warps' fragments, one half (rows 0..7) or two
+      const int halves = tall ? 2 : 1;
+      float2* mine = red.sum + (buf * kConsumerWarps + cw) * halves * lanes;
+      float part[4];
+      switch (form) {
+        case FORM_ROWS4: shrink_partials<FORM_ROWS4>(acc, part); break;
+        case FORM_ROWS8: shrink_partials<FORM_ROWS8>(acc, part); break;
+        default: shrink_partials<FORM_FULL>(acc, part); break;
       }
+      if (lane < lanes) mine[lane] = make_float2(part[0], part[1]);
+      if (tall) mine[32 + lane] = make_float2(part[2], part[3]);
       __syncwarp();
       int old = 0;
       if (lane == 0) {
@@ -825,22 +878,30 @@ __device__ __forceinline__ void shrink_consumer(const ShrinkArgs& a, const unsig
       old = __shfl_sync(FULL_MASK, old, 0);
       if (old == kConsumerWarps - 1) {
         __threadfence_block();
-        const int j = lane / nt, i = lane - j * nt;  // red_row index = row * nt + token
-        if (lane < (wide ? kWideRows : kMaxRows) * nt) {
-          float sum = 0.f;
+        for (int h = 0; h < halves; ++h) {
+          float2 sum = make_float2(0.f, 0.f);
 #pragma unroll
-          for (int w = 0; w < kConsumerWarps; ++w) sum += red.sum[buf][w][lane];
-          if (j < nrows && i < n && m[3] + j < a.delta_width) {
-            if (a.tp.enabled) {
-              // tensor parallelism: this rank's rows go straight into every rank's delta buffer (NVLink stores)
-              const int64_t R = static_cast<int64_t>(a.tp.n_parts) * a.delta_width;
-              const int64_t at = ((static_cast<int64_t>(tp_slot) * 3 + m[4]) * a.tp.full_tokens + m[8 + i]) * R +
-                                 static_cast<int64_t>(a.tp.my_part) * m[7] + m[3] + j;
-              const T v = from_f32<T>(sum);
-              for (int g = 0; g < a.tp.n_parts; ++g) reinterpret_cast<T*>(a.tp.full[g])[at] = v;
-            } else {
-              T* d = reinterpret_cast<T*>(pick3(a.delta, m[4]));
-              d[static_cast<int64_t>(m[8 + i]) * a.delta_stride + m[3] + j] = from_f32<T>(sum);
+          for (int w = 0; w < kConsumerWarps; ++w) {
+            const float2 v = red.sum[((buf * kConsumerWarps + w) * halves + h) * lanes + (lane & (lanes - 1))];
+            sum.x += v.x;
+            sum.y += v.y;
+          }
+          const int j = 8 * h + (lane >> 2);
+#pragma unroll
+          for (int q = 0; q < 2; ++q) {
+            const int i = 2 * (lane & 3) + q;
+            if (j < nrows && i < n && m0.w + j < a.delta_width) {
+              const T v = from_f32<T>(q == 0 ? sum.x : sum.y);
+              if (a.tp.enabled) {
+                // tensor parallelism: this rank's rows go straight into every rank's delta buffer (NVLink stores)
+                const int64_t R = static_cast<int64_t>(a.tp.n_parts) * a.delta_width;
+                const int64_t at = ((static_cast<int64_t>(tp_slot) * 3 + m1.x) * a.tp.full_tokens + m[8 + i]) * R +
+                                   static_cast<int64_t>(a.tp.my_part) * m1.w + m0.w + j;
+                for (int p = 0; p < a.tp.n_parts; ++p) reinterpret_cast<T*>(a.tp.full[p])[at] = v;
+              } else {
+                T* d = reinterpret_cast<T*>(pick3(a.delta, m1.x));
+                d[static_cast<int64_t>(m[8 + i]) * a.delta_stride + m0.w + j] = v;
+              }
             }
           }
         }
@@ -889,7 +950,7 @@ __global__ void __launch_bounds__(kPipeThreads, kPipeCtasPerSm) lora_shrink_pipe
   // by thread: see TpLink::inband)
   if (!(a.tp.enabled && a.tp.inband >= 2)) pdl_launch_dependents();
   if (EXACT) {
-    fill_item_counts(a.src, a.tb, ctl, tid, [&](int rr, int n) { return shrink_items_of(a, rr, n); });
+    fill_item_counts(a.src, a.tb, ctl, tid, [&](int rr, int) { return shrink_items_of(a, rr); });
     __syncthreads();
   }
   if (warp < kProducerWarps) {
@@ -932,7 +993,6 @@ __device__ __forceinline__ void expand_producer(const ExpandArgs& a, unsigned ch
   const T* w = reinterpret_cast<const T*>(a.w);
   const int64_t G = gridDim.x;
   const uint32_t ring_base = smem_u32(ring_mem);
-  PipeCtl::Prod& pp = c.prod[role];
   Ring r;
   r.role = role;
   r.cap = EXACT ? kExpandRingBytes : kRingBytes;  // see kExpandRingBytes
@@ -943,116 +1003,123 @@ __device__ __forceinline__ void expand_producer(const ExpandArgs& a, unsigned ch
   if (a.tp.enabled && a.tp.inband == 3) {
     const int e = *reinterpret_cast<volatile const int32_t*>(a.tp.seq_state + 1);  // left by this exchange's shrink
     delta_off = (e % 3) * 3 * a.tp.full_tokens * a.delta_stride;
-    if (blockIdx.x == 0 && lane == 0) a.tp.seq_state[0] = e + 1;  // the next shrink reads it after its own wait
+    if (blockIdx.x == 0 && lane == 0 && role == 0) a.tp.seq_state[0] = e + 1;  // the next shrink reads it after its own wait
   }
   auto rank_ok = [&](int rk) { return expand_rank_ok(a, rk); };
   auto chunks_of = [&](int p, int rk) { return expand_chunks_of(a, p, rk); };
-  const ItemMap map = EXACT ? build_item_map(a.src, total_chunks, c, lane, [&](int rr, int) { return expand_items_of(a, rr); })
+  const ItemMap map = EXACT ? build_item_map(a.src, total_chunks, c, lane, role, [&](int rr, int) { return expand_items_of(a, rr); })
                             : padded_item_map(a.src, total_chunks);
   const int mode = EXACT ? map.mode : 0;
   int64_t n_items = map.n_items;
 
-  for (int64_t batch0 = blockIdx.x; batch0 < n_items && !r.dead; batch0 += 32 * G) {
-    // d_i[lane] = {pr0, n, r, p, clen, first output, scale bits, chunk start inside pool row pr0, tok[8]},
-    // d_l[lane][j] = pool row of slot row pr0 + j
-    const int64_t item = batch0 + lane * G;
-    int valid = 0;
-    if (item < n_items) {
-      int tile, ch;
-      item_to_tile(map, c, item, tile, ch);
-      // projection and chunk: known before the tile record arrives unless ranks are mixed
-      int p = 0;
-      auto split = [&](int rk) {
-        while (p + 1 < a.nproj && ch >= chunks_of(p, rk)) {
-          ch -= chunks_of(p, rk);
-          ++p;
+  // (a producer warp whose wait ran out goes on meeting the other one)
+  for (int64_t batch0 = blockIdx.x; batch0 < n_items; batch0 += 32 * G) {
+    producers_sync();
+    // d_i[lane] = {log2 r, n, r, p, clen, first output, scale bits, chunk start inside its first pool row, tok[8]},
+    // d_l[lane][j] = pool row of the chunk's j-th slot row
+    if (role == 0) {
+      const int64_t item = batch0 + lane * G;
+      int valid = 0;
+      if (item < n_items) {
+        int tile, ch;
+        item_to_tile(map, a.per_tile, c, item, tile, ch);
+        // projection and chunk: known before the tile record arrives unless ranks are mixed
+        int p = 0;
+        auto split = [&](int rk) {
+          while (p + 1 < a.nproj && ch >= chunks_of(p, rk)) {
+            ch -= chunks_of(p, rk);
+            ++p;
+          }
+        };
+        if (mode == 0) {
+          while (p + 1 < a.nproj && ch >= a.chunk_begin[p + 1]) ++p;
+          ch -= a.chunk_begin[p];
+        } else if (mode == 1 && rank_ok(map.uniform * a.rank_mult)) {
+          split(map.uniform * a.rank_mult);
         }
-      };
-      if (mode == 0) {
-        while (p + 1 < a.nproj && ch >= a.chunk_begin[p + 1]) ++p;
-        ch -= a.chunk_begin[p];
-      } else if (mode == 1 && rank_ok(map.uniform * a.rank_mult)) {
-        split(map.uniform * a.rank_mult);
-      }
-      // resolved tiles: where projection and chunk follow from the item index alone, the chunk's pool rows and the
-      // adapter's scale are fetched now, together with the header and the record that will say whether they count
-      int spec_row[kSpanRows], spec_scale = 0;
-      bool spec = false;
-      if (a.src.mode == MODE_PLAN && a.src.xoff > 0 && mode != 2) {
-        const int32_t* xt = a.src.plan + a.src.xoff + static_cast<int64_t>(tile) * (kXtHead + 4 * a.src.xrcap);
-        const int qk_s = pick3(a.qkvo, p);
-        const int pr_s = static_cast<int>(static_cast<int64_t>(ch) * kPipeChunk / S);
-        spec_scale = xt[8];
+        // resolved tiles: where projection and chunk follow from the item index alone, the chunk's pool rows are
+        // fetched now, together with the header and the record that will say whether they count
+        const bool entry = a.src.mode == MODE_PLAN && a.src.xoff > 0;
+        int64_t row[kSpanRows];
+        auto fetch_rows = [&](int qk, int pr) {
+          const int32_t* xt = a.src.plan + a.src.xoff + static_cast<int64_t>(tile) * (kXtHead + 4 * a.src.xrcap) + kXtHead +
+                              qk * a.src.xrcap;
 #pragma unroll
-        for (int j = 0; j < kSpanRows; ++j)
-          spec_row[j] = xt[kXtHead + qk_s * a.src.xrcap + min(pr_s + j, a.src.xrcap - 1)];
-        spec = true;
-      }
-      TileInfo t;
-      if (lookup_tile(a.src, a.tb, tile, t, a.status)) {
-        const int rk = t.r * a.rank_mult;
-        if (mode == 2 && rank_ok(rk)) split(rk);
-        const int h_out = pick3(a.h_out, p);
-        const int64_t flat_total = static_cast<int64_t>(h_out) * rk;
-        const int64_t c0 = static_cast<int64_t>(ch) * kPipeChunk;
-        if (c0 < flat_total) {
-          if (!rank_ok(rk)) {
-            set_status(a.status, SLORA_STATUS_BAD_RANK);
-          } else {
-            const int clen = static_cast<int>(min(static_cast<int64_t>(kPipeChunk), flat_total - c0));
-            const int qk = pick3(a.qkvo, p);
-            const int64_t pr0 = c0 / S, pr1 = (c0 + clen - 1) / S;
-            bool ok = pr1 - pr0 < kSpanRows && pr1 < t.r;
-            if (ok) {
+          for (int j = 0; j < kSpanRows; ++j) row[j] = xt[min(pr + j, a.src.xrcap - 1)];
+        };
+        if (entry && mode != 2) fetch_rows(pick3(a.qkvo, p), a.stride.div(min(ch, 0x7fffffff / kPipeChunk) * kPipeChunk));
+        TileInfo t;
+        if (lookup_tile(a.src, a.tb, tile, t, a.status)) {
+          const int rk = t.r * a.rank_mult;
+          if (mode == 2 && rank_ok(rk)) split(rk);
+          const int h_out = pick3(a.h_out, p);
+          const int64_t flat_total = static_cast<int64_t>(h_out) * rk;
+          const int64_t c0 = static_cast<int64_t>(ch) * kPipeChunk;
+          if (c0 < flat_total) {
+            if (!rank_ok(rk)) {
+              set_status(a.status, SLORA_STATUS_BAD_RANK);
+            } else {
+              const int clen = static_cast<int>(min(static_cast<int64_t>(kPipeChunk), flat_total - c0));
+              const int qk = pick3(a.qkvo, p);
+              const int pr0 = a.stride.div(static_cast<int>(c0)), pr1 = a.stride.div(static_cast<int>(c0) + clen - 1);
+              bool ok = pr1 - pr0 < kSpanRows && pr1 < t.r;
+              if (ok) {
+                if (!t.xok) {
 #pragma unroll
-              for (int j = 0; j < kSpanRows; ++j) {
-                if (pr0 + j <= pr1) {
-                  const int64_t e = (spec && t.xok) ? spec_row[j] : tile_loc(t, a.tb, qk, pr0 + j);
-                  if (e < 0 || e >= a.tb.pool_rows) ok = false;
-                  pp.d_l[lane][j] = e;
+                  for (int j = 0; j < kSpanRows; ++j) row[j] = tile_loc(t, a.tb, qk, min(pr0 + j, pr1));
+                } else if (mode == 2) {
+                  fetch_rows(qk, pr0);
+                }
+#pragma unroll
+                for (int j = 0; j < kSpanRows; ++j) {
+                  if (pr0 + j <= pr1) {
+                    if (row[j] < 0 || row[j] >= a.tb.pool_rows) ok = false;
+                    c.d_l[lane][j] = static_cast<int32_t>(row[j]);  // (pool_rows < 2^31 here)
+                  }
                 }
               }
-            }
-            if (ok) {
+              if (ok) {
+                int tok[kTileTokens];
 #pragma unroll
-              for (int i = 0; i < kTileTokens; ++i) pp.d_i[lane][8 + i] = i < t.n ? tile_token(t, i) : 0;
-              pp.d_i[lane][0] = static_cast<int>(pr0);
-              pp.d_i[lane][1] = t.n;
-              pp.d_i[lane][2] = rk;
-              pp.d_i[lane][3] = p;
-              pp.d_i[lane][4] = clen;
-              pp.d_i[lane][5] = static_cast<int>(c0 / rk);
-              {
+                for (int i = 0; i < kTileTokens; ++i) tok[i] = i < t.n ? tile_token(t, i) : 0;
+                const int lg = 31 - __clz(rk);  // rk is a power of two (rank_ok)
                 // the scale's 16 bits: from the resolved tile when it counts and carries one, else from the table
                 T sc;
-                if (spec && t.xok && (spec_scale & 0x10000)) {
-                  const unsigned short bits = static_cast<unsigned short>(spec_scale & 0xffff);
+                if (t.xok && (t.xscale & 0x10000)) {
+                  const unsigned short bits = static_cast<unsigned short>(t.xscale & 0xffff);
                   sc = *reinterpret_cast<const T*>(&bits);
                 } else {
                   sc = reinterpret_cast<const T*>(a.scales)[t.adapter];
                 }
-                pp.d_i[lane][6] = __float_as_int(to_f32<T>(sc));
+                int4* di = reinterpret_cast<int4*>(c.d_i[lane]);
+                di[0] = make_int4(lg, t.n, rk, p);
+                di[1] = make_int4(clen, static_cast<int>(c0) >> lg, __float_as_int(to_f32<T>(sc)),
+                                  static_cast<int>(c0 - static_cast<int64_t>(pr0) * S));
+                di[2] = make_int4(tok[0], tok[1], tok[2], tok[3]);
+                di[3] = make_int4(tok[4], tok[5], tok[6], tok[7]);
+                valid = 1;
+              } else {
+                set_status(a.status, SLORA_STATUS_BAD_TABLE);
               }
-              pp.d_i[lane][7] = static_cast<int>(c0 - pr0 * S);  // chunk start inside its first pool row
-              valid = 1;
-            } else {
-              set_status(a.status, SLORA_STATUS_BAD_TABLE);
             }
           }
         }
       }
+      const uint32_t mask = __ballot_sync(FULL_MASK, valid != 0);
+      if (lane == 0) c.valid_mask = mask;
     }
-    const uint32_t valid_mask = __ballot_sync(FULL_MASK, valid != 0);
-    __syncwarp();
+    producers_sync();
+    const uint32_t valid_mask = c.valid_mask;
 
-    // one copy per lane: 0..15 pieces of the B chunk, 16..23 y segments, 24..31 delta rows.  Everything that does
+    // one copy per lane: 0..5 the B chunk's pool rows, 16..23 y segments, 24..31 delta rows.  Everything that does
     // not depend on where the stage lands in the ring is worked out BEFORE the wait for ring space: what follows the
     // wait is on the path from a consumer's release of a stage to the next copy's issue.
     for (uint32_t left = valid_mask; left != 0 && !r.dead; left &= left - 1) {
       const int k = __ffs(left) - 1;
-      const int* di = pp.d_i[k];
-      const int n = di[1], rk = di[2], p = di[3], clen = di[4], obase = di[5];
-      const int nout = clen / rk;
+      const int* di = c.d_i[k];
+      const int4 d0 = *reinterpret_cast<const int4*>(di), d1 = *reinterpret_cast<const int4*>(di + 4);
+      const int n = d0.y, rk = d0.z, p = d0.w, clen = d1.x, obase = d1.y, m_scale = d1.z, col0 = d1.w;
+      const int nout = clen >> d0.x;
       const uint32_t b_bytes = static_cast<uint32_t>(clen) * sizeof(T);
       const uint32_t y_bytes = static_cast<uint32_t>(nout) * sizeof(T);
       const uint32_t d_bytes = static_cast<uint32_t>(rk) * sizeof(T);
@@ -1062,16 +1129,16 @@ __device__ __forceinline__ void expand_producer(const ExpandArgs& a, unsigned ch
       uint32_t rel = 0, bytes = 0;  // this lane's copy: offset inside the stage, size
       const T* src = w;
       bool is_act = false;
-      if (lane < kMaxPieces) {
-        const int poff = lane * a.piece;
-        if (poff < clen) {
-          const int f = di[7] + poff;  // offset from the start of the chunk's first pool row
-          const int pr = f / static_cast<int>(S), col = f - pr * static_cast<int>(S);
-          src = w + pp.d_l[k][pr] * S + col;
+      if (lane < kSpanRows) {
+        // the chunk's part of pool row pr0 + lane: one copy per pool row, whole rows except at the chunk's ends
+        const int64_t start = lane * S - col0;  // (before the chunk for row 0)
+        if (start < clen) {
+          const int poff = max(static_cast<int>(start), 0), col = lane == 0 ? col0 : 0;
+          src = w + c.d_l[k][lane] * S + col;
           rel = static_cast<uint32_t>(poff) * sizeof(T);
-          bytes = static_cast<uint32_t>(min(a.piece, clen - poff)) * sizeof(T);
+          bytes = static_cast<uint32_t>(min(static_cast<int>(S) - col, clen - poff)) * sizeof(T);
         }
-      } else if (lane < 16 + n) {
+      } else if (lane >= 16 && lane < 16 + n) {
         src = reinterpret_cast<const T*>(pick3(a.y, p)) + static_cast<int64_t>(mytok) * pick3(a.y_stride, p) + obase;
         rel = b_bytes + static_cast<uint32_t>(lane - 16) * y_bytes;
         bytes = y_bytes;
@@ -1082,28 +1149,24 @@ __device__ __forceinline__ void expand_producer(const ExpandArgs& a, unsigned ch
         bytes = d_bytes;
         is_act = true;
       }
-      const int m_scale = di[6];
       const uint32_t off = ring_alloc(r, c, sz, lane);
       if (r.dead) break;
       const uint32_t slot = r.g % kSlots;
-      const bool mine = static_cast<int>(r.g % kProducerWarps) == role;
       r.head = off + sz;
-      if (lane == 0) pp.off[slot] = off;
-      if (!mine) {
-        __syncwarp();
-        ring_issue(r, c, slot, 0, nullptr, 0u, false, lane);
-        continue;
+      if (lane == 0) c.off[role][slot] = off;
+      if (role == 0) {
+        if (lane == 0) {  // the stage record in two 16-byte stores
+          int4* mrec = reinterpret_cast<int4*>(c.meta[slot]);
+          mrec[0] = make_int4(0, n, rk, p);
+          mrec[1] = make_int4(clen, obase, m_scale, static_cast<int>(off));
+        } else if (lane >= kActLane && lane < kActLane + kTileTokens) {
+          c.meta[slot][8 + lane - kActLane] = mytok;
+        }
+        __syncwarp();  // the arrive below publishes every lane's part of the stage record
+        if (lane == 0) mbar_expect_tx(&c.full[slot], total);
       }
-      if (lane == 0) {  // the stage record in two 16-byte stores
-        int4* mrec = reinterpret_cast<int4*>(c.meta[slot]);
-        mrec[0] = make_int4(0, n, rk, p);
-        mrec[1] = make_int4(clen, obase, m_scale, static_cast<int>(off));
-      } else if (lane >= 16 && lane < 24) {
-        c.meta[slot][8 + lane - 16] = mytok;
-      }
-      __syncwarp();  // the arrive below publishes every lane's part of the stage record
-      if (lane == 0) mbar_expect_tx(&c.full[slot], total);
-      ring_issue(r, c, slot, ring_base + off + rel, src, bytes, is_act, lane);
+      if (role != 0) ring_enter(r, lane);
+      ring_issue(r, c, slot, ring_base + off + rel, src, is_act == (role != 0) ? bytes : 0u);
     }
     __syncwarp();
     if (!EXACT && a.src.mode == MODE_PLAN) n_items = padded_item_count(a.src, total_chunks);
@@ -1153,59 +1216,64 @@ __device__ __noinline__ void expand_settle_slow(T* ds, const int* m, int r, cons
   __syncwarp();
 }
 
-// One consumer warp's part of an expand stage.  LPO = lanes per output = r / 8.  The warp owns flat elements
-// [cw*2048, +2048) of the chunk as 8 loads of 256 elements; load m, lane l holds the 8 values of output
-// (cw*8 + m)*(32/LPO) + l/LPO for k in [(l % LPO)*8, +8).
-template <typename T, int LPO, bool FULL, bool INBAND = false>
+// One consumer warp's part of an expand stage of rank R and at most NT tokens: flat elements [cw * 2048, +2048) of the
+// chunk on the tensor pipe (expand_group), then y = y + scale * v with y read from the stage as vectors and written
+// back as vectors.
+template <typename T, int R, int NT, bool INBAND>
 __device__ __forceinline__ void expand_stage(const T* bs, const int* m, T* y, int64_t y_stride, int lane, int cw,
-                                             const T* dglobal = nullptr, int64_t dglobal_stride = 0,
-                                             int32_t* status = nullptr, volatile int* gave_up = nullptr) {
-  constexpr int OPL = 32 / LPO;
-  constexpr int NV = LPO >= 8 ? 1 : 8 / LPO;
-  constexpr int R = LPO * 8;
-  constexpr int SPAN = kPipeChunk / kConsumerWarps;  // 2048
+                                             const T* dglobal, int64_t dglobal_stride, int32_t* status,
+                                             volatile int* gave_up) {
+  using S = ExpandShape<R, false>;
+  using K = TokenSplit<NT>;
   const int n = m[1], clen = m[4], obase = m[5];
-  if (cw * SPAN >= clen) return;
+  if (cw * (kPipeChunk / kConsumerWarps) >= clen) return;
   const int nout = clen / R;
   const float scale = __int_as_float(m[6]);
   const T* ys = bs + clen;
   const T* ds = ys + n * nout;
-  uint4 bv[8];
-#pragma unroll
-  for (int mm = 0; mm < 8; ++mm) {
-    const int foff = cw * SPAN + mm * 256 + lane * 8;
-    bv[mm] = (FULL || foff < clen) ? *reinterpret_cast<const uint4*>(bs + foff) : make_uint4(0u, 0u, 0u, 0u);
-  }
-  // in-band signalling: have this stage's delta values all arrived?  (after the B loads have been issued, so that the
-  // look costs no latency of its own)
+  // in-band signalling: have this stage's delta values all arrived?
   if (INBAND) expand_settle_delta<T>(const_cast<T*>(ds), m, R, dglobal, dglobal_stride, status, gave_up, lane);
-  const int kp = (lane & (LPO - 1)) * 8;
-  const int g = lane / LPO;
-  const int m_base = expand_m_base<LPO>(lane);
-  const bool writer = (LPO < 16) || ((lane & 8) == 0);
-  int o_loc[NV];
+  const int g = lane >> 2, t = lane & 3;
+  const DeltaFrag<R> f = load_delta_frag<T, R>(ds, K::column(g, n), t);
+  const int tok0 = K::tok0(t);
+  const int x = expand_x<R, false>(g);
+  constexpr int ROUNDS = (S::NG + K::DUP - 1) / K::DUP;
+#pragma unroll 1
+  for (int r = 0; r < ROUNDS; ++r) {
+    float acc[S::NBLK][2];
+    expand_round<T, R, false, NT>(acc, bs, f, cw, r, nout, lane);
+    const int gr = r * K::DUP + K::di(t);
+    const int o = expand_out<R, false>(cw, gr, g);
+    const bool live = gr < S::NG && o < nout;
 #pragma unroll
-  for (int i = 0; i < NV; ++i) o_loc[i] = (cw * 8 + m_base + i) * OPL + g;  // output index inside the chunk
+    for (int c = 0; c < K::TPL; ++c) {
+      float v[S::VPL], yv[S::VPL];
+#pragma unroll
+      for (int i = 0; i < S::VPL; ++i) v[i] = acc[i][c];
+      xor_index(v, x);
+      const int tok = tok0 + c;
+      if (live && tok < n) {
+        load_vec<T>(yv, ys + tok * nout + o);
+#pragma unroll
+        for (int i = 0; i < S::VPL; ++i) yv[i] = fmaf(scale, v[i], yv[i]);
+        store_vec<T>(y + static_cast<int64_t>(m[8 + tok]) * y_stride + obase + o, yv);
+      }
+    }
+  }
+}
 
-  for (int tt = 0; tt < n; ++tt) {
-    const uint4 dv = *reinterpret_cast<const uint4*>(ds + tt * R + kp);
-    float yv[NV];
-#pragma unroll
-    for (int i = 0; i < NV; ++i) {
-      yv[i] = (FULL || (writer && o_loc[i] < nout)) ? to_f32<T>(ys[tt * nout + o_loc[i]]) : 0.f;
-    }
-    float v[8];
-#pragma unroll
-    for (int mm = 0; mm < 8; ++mm) {
-      v[mm] = 0.f;
-      dot8<T>(v[mm], bv[mm], dv);
-    }
-    expand_butterfly<LPO>(v, lane);
-    T* yrow = y + static_cast<int64_t>(m[8 + tt]) * y_stride + obase;
-#pragma unroll
-    for (int i = 0; i < NV; ++i) {
-      if (writer && (FULL || o_loc[i] < nout)) yrow[o_loc[i]] = from_f32<T>(fmaf(scale, v[i], yv[i]));
-    }
+template <typename T, int R, bool INBAND>
+__device__ __forceinline__ void expand_stage_tokens(const T* bs, const int* m, T* y, int64_t y_stride, int lane, int cw,
+                                                    const T* dg, int64_t dgs, int32_t* status, volatile int* gave_up) {
+  const int n = m[1];
+  if (n <= 1) {
+    expand_stage<T, R, 1, INBAND>(bs, m, y, y_stride, lane, cw, dg, dgs, status, gave_up);
+  } else if (n <= 2) {
+    expand_stage<T, R, 2, INBAND>(bs, m, y, y_stride, lane, cw, dg, dgs, status, gave_up);
+  } else if (n <= 4) {
+    expand_stage<T, R, 4, INBAND>(bs, m, y, y_stride, lane, cw, dg, dgs, status, gave_up);
+  } else {
+    expand_stage<T, R, 8, INBAND>(bs, m, y, y_stride, lane, cw, dg, dgs, status, gave_up);
   }
 }
 
@@ -1231,22 +1299,12 @@ __device__ __forceinline__ void expand_consumer(const ExpandArgs& a, const unsig
     const int64_t ystr = pick3(a.y_stride, p);
     const T* dg = INBAND ? reinterpret_cast<const T*>(pick3(a.delta, p)) + delta_off : nullptr;
     const int64_t dgs = a.delta_stride;
-    if (m[4] == kPipeChunk) {  // complete chunk: no bounds checks
-      switch (m[2]) {
-        case 8: expand_stage<T, 1, true, INBAND>(bs, m, y, ystr, lane, cw, dg, dgs, a.status, &c.tp_gave_up); break;
-        case 16: expand_stage<T, 2, true, INBAND>(bs, m, y, ystr, lane, cw, dg, dgs, a.status, &c.tp_gave_up); break;
-        case 32: expand_stage<T, 4, true, INBAND>(bs, m, y, ystr, lane, cw, dg, dgs, a.status, &c.tp_gave_up); break;
-        case 64: expand_stage<T, 8, true, INBAND>(bs, m, y, ystr, lane, cw, dg, dgs, a.status, &c.tp_gave_up); break;
-        default: expand_stage<T, 16, true, INBAND>(bs, m, y, ystr, lane, cw, dg, dgs, a.status, &c.tp_gave_up); break;
-      }
-    } else {
-      switch (m[2]) {
-        case 8: expand_stage<T, 1, false, INBAND>(bs, m, y, ystr, lane, cw, dg, dgs, a.status, &c.tp_gave_up); break;
-        case 16: expand_stage<T, 2, false, INBAND>(bs, m, y, ystr, lane, cw, dg, dgs, a.status, &c.tp_gave_up); break;
-        case 32: expand_stage<T, 4, false, INBAND>(bs, m, y, ystr, lane, cw, dg, dgs, a.status, &c.tp_gave_up); break;
-        case 64: expand_stage<T, 8, false, INBAND>(bs, m, y, ystr, lane, cw, dg, dgs, a.status, &c.tp_gave_up); break;
-        default: expand_stage<T, 16, false, INBAND>(bs, m, y, ystr, lane, cw, dg, dgs, a.status, &c.tp_gave_up); break;
-      }
+    switch (m[2]) {
+      case 8: expand_stage_tokens<T, 8, INBAND>(bs, m, y, ystr, lane, cw, dg, dgs, a.status, &c.tp_gave_up); break;
+      case 16: expand_stage_tokens<T, 16, INBAND>(bs, m, y, ystr, lane, cw, dg, dgs, a.status, &c.tp_gave_up); break;
+      case 32: expand_stage_tokens<T, 32, INBAND>(bs, m, y, ystr, lane, cw, dg, dgs, a.status, &c.tp_gave_up); break;
+      case 64: expand_stage_tokens<T, 64, INBAND>(bs, m, y, ystr, lane, cw, dg, dgs, a.status, &c.tp_gave_up); break;
+      default: expand_stage_tokens<T, 128, INBAND>(bs, m, y, ystr, lane, cw, dg, dgs, a.status, &c.tp_gave_up); break;
     }
     __syncwarp();
     if (lane == 0) mbar_arrive(&c.empty[slot]);
