@@ -129,13 +129,17 @@ def check(rc: int) -> None:
         raise RuntimeError(f"slora_b200: {last_error()} (status {rc})")
 
 
+_DTYPE_CODES = {}
+
+
 def dtype_code(torch_dtype) -> int:
-    import torch
-    if torch_dtype == torch.float16:
-        return F16
-    if torch_dtype == torch.bfloat16:
-        return BF16
-    raise RuntimeError(f"No suitable kernel. dtype={torch_dtype}")
+    if not _DTYPE_CODES:
+        import torch
+        _DTYPE_CODES.update({torch.float16: F16, torch.bfloat16: BF16})
+    code = _DTYPE_CODES.get(torch_dtype)
+    if code is None:
+        raise RuntimeError(f"No suitable kernel. dtype={torch_dtype}")
+    return code
 
 
 def ptr(t) -> int:
@@ -150,5 +154,7 @@ def require_cuda(*tensors) -> None:
 
 
 def current_stream_ptr() -> int:
-    import torch
-    return torch.cuda.current_stream().cuda_stream
+    """The current device's current stream.  ``torch.cuda.current_stream()`` builds a Stream object (3.2 us on the host
+    of a B200 box, a third of a call's time in Python); the raw query behind it takes a tenth of that."""
+    from torch import _C
+    return _C._cuda_getCurrentRawStream(_C._cuda_getDevice())
