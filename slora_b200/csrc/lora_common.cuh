@@ -22,7 +22,8 @@ constexpr uint32_t kSpinLimit = 1u << 18;
 // tile record: {adapter, first slot in perm, tokens (0 = skip), slot_rows r, first loc entry, big, 0, 0}
 //   big = 1 when the tile's adapter has kBigGroupTokens tokens or more in the batch and 8..128 slot rows (a multiple
 //   of 8): such groups are also listed as big tiles of up to 128 tokens for the tensor-core kernels
-// big-tile record: {adapter, first slot in perm, tokens, slot_rows r, first loc entry, 0, 0, 0}
+// big-tile record: {adapter, first slot in perm, tokens, slot_rows r, first loc entry, 1 when the tokens are consecutive,
+//   the first of them, 1 when the group is in the batch's order}
 constexpr int PH_MAGIC = 0, PH_NTILES = 1, PH_STATUS = 2, PH_MAXTILES = 3, PH_T = 4, PH_NADAPTERS = 5, PH_NBIG = 6,
               PH_BIGOFF = 7, PH_MAXBIG = 8, PH_UNIFORM = 9;  // PH_UNIFORM: the slot rows every non-empty tile has, 0 when they differ
 // PH_NSMALL: 8-token tiles of groups that are not big (the CUDA-core kernels' share when big groups go to the tensor
@@ -41,6 +42,7 @@ constexpr int kXtHead = 12;
 constexpr int kBigGroupTokens = 128;  // planned batches: same-adapter groups at least this long go to the tensor cores
 constexpr int kBigSegmentTokens = 32;  // segment calls: segments at least this long do
 constexpr int kBigTileTokens = 128;
+constexpr int kOrderedGroups = 64;  // big groups whose tokens the plan keeps in the batch's order
 constexpr int PH_WORDS = 16;
 constexpr int kTileWords = 8;
 constexpr int32_t kPlanMagic = 0x534c5034;  // "SLP4"
@@ -183,7 +185,7 @@ struct ExpandArgs {
   int max_rank;  // widest rank the delta buffers hold (delta_width * delta_parts): wider adapters are refused
   int piece;  // simple kernel: elements per bulk copy (power of two dividing pool_stride, <= kChunk)
   FastDiv per_tile;  // pipelined kernel: items enumerated per tile (padded enumeration)
-  FastDiv stride;    // pipelined kernel: elements per pool row
+  FastDiv stride;    // pipelined and tensor-core kernels: elements per pool row
   int mma_stage_bytes;  // tensor-core kernel: bytes of one operand tile [128 x kpad_max]
   TpLink tp;
   int32_t* status;

@@ -809,6 +809,7 @@ int run_expand(const TileSrc& src, const Tables& tb, const void* w, const void* 
   can_mma = can_mma && tb.pool_stride < 0x7fffffff && src.T < 0x7fffffff;
   if (can_mma) {
     ExpandArgs m = a;
+    m.stride = make_fast_div(static_cast<uint32_t>(tb.pool_stride));
     m.src.seg_split = src.seg_split;
     m.src.mma_max_rows = delta_width < kMmaMaxRank ? delta_width : kMmaMaxRank;
     m.chunk_begin[0] = 0;

@@ -15,11 +15,18 @@
 //            that one lane adds into y with a TMA reduce (an element-wise 16-bit add in L2, which is also how the
 //            reference accumulates: it rounds the FP32 sum to the output type and then adds, bgmv_impl.cuh:185-199).
 //
-// Operand layouts in shared memory.  Gathered operands (adapter rows, B chunks, delta tile) use the un-swizzled
+// What bounds them (measured on B200, clock64 in every phase): the loaders' instructions.  A 16-byte cp.async that
+// touches 8 rows x 64 bytes, with the row offset read from shared memory between two copies, took 280 cycles a warp
+// instruction; eight lanes on the 128 bytes of one row and eight addresses worked out ahead brought the shrink of 32 tiles
+// (q, k, v; 4096 tokens, hidden 4096) from 21.4 to 17.3 us, and with consecutive tokens moved as whole tiles to 15.7.  The
+// expand (46.2 -> 44.9 us, 201 MB of y read and written) waits for the copy engine's 16-bit adds: adding to y in the
+// epilogue instead took 63 us, four loader warps with a chunk ahead 48.5.
+//
+// Operand layouts in shared memory.  The expand's gathered operands (B chunks, delta tile) use the un-swizzled
 // K-major core-matrix layout: the tile [rows x 8*chunks] is cut into 16-byte chunks (8 elements of K); chunk
 // (row, c) lives at c * rows * 16 + row * 16, so eight consecutive rows of one chunk form a contiguous 128-byte
 // core matrix, the descriptor's stride between 8-row groups (SBO) is 128 bytes and the stride between the two
-// K-chunks of one K=16 instruction (LBO) is rows * 16 bytes.  TMA-loaded activations use the 128-byte swizzled
+// K-chunks of one K=16 instruction (LBO) is rows * 16 bytes.  The shrink's operands use the 128-byte swizzled
 // K-major layout (rows of 64 elements, SBO = 1024 bytes, K advanced by 32 bytes inside the swizzle span).
 //
 // Every wait is bounded; a CTA that gives up records SLORA_STATUS_TIMEOUT and frees its tensor memory before it
@@ -267,6 +274,10 @@ __device__ __forceinline__ bool lookup_mma_tile(const TileSrc& s, const Tables& 
     t.r = r0.w;
     t.loc_base = r1.x;
     t.perm = s.plan + PH_WORDS + kTileWords * hdr[PH_MAXTILES];
+    if (r1.y != 0) {  // consecutive tokens: whole tiles can be moved
+      t.perm = nullptr;
+      t.first = r1.z;
+    }
     return t.n > 0 && t.r > 0 && tb.pool_stride % t.r == 0 && t.r <= s.mma_max_rows;
   }
   t.perm = nullptr;
@@ -300,7 +311,7 @@ __device__ __forceinline__ bool lookup_mma_tile(const TileSrc& s, const Tables& 
 // ------------------------------------------------------------------------------------------------------------
 // shrink: delta[p][tok, j] = sum_k x[tok, k] * A_p[j, k] for the projections p of this CTA's group
 // grid: (segment tile, projection group).  dynamic shared memory (1024-byte aligned): `mma_stages` stages of
-//   [x tile 128 x 64, swizzled][adapter rows npad_max x 64, core-matrix layout]
+//   [x tile 128 x 64][adapter rows npad_max x 64], both swizzled
 // ------------------------------------------------------------------------------------------------------------
 struct ShrinkMmaCtl {
   uint64_t full[kMmaMaxStages];   // arrivals: the stage's loader warp and, for consecutive tokens, the activation
@@ -387,10 +398,25 @@ __global__ void __launch_bounds__(kMmaShrinkThreads, 1)
   if (warp < kMmaLoaderWarps) {
     // ---- loader warp: gathers the adapter rows of K-blocks warp, warp + nst, ... into stage `warp` ----
     if (warp < nst) {
-      const int row_lo = lane & 7, c_lo = lane >> 3;
+      // eight lanes copy the 128 bytes of one row (whole lines, and no bank twice), eight rows' addresses are worked out
+      // before the first of their copies is issued (a copy is an ordering point for the compiler)
+      const int row_lo = lane >> 3, c = lane & 7;
       const T* w = reinterpret_cast<const T*>(a.w);
       const T* x = reinterpret_cast<const T*>(a.x);
-      const uint32_t dst0 = smem0 + warp * stage_bytes + kMmaXTileBytes + row_lo * 16;
+      // both operands in the 128-byte swizzled layout: chunk c of row i at i * 128 + ((c ^ (i & 7)) << 4)
+      const uint32_t xdst = smem0 + warp * stage_bytes, wdst = xdst + kMmaXTileBytes;
+      auto copy_rows = [&](const T* src, const int64_t* off, uint32_t dst, int n_rows, int k0) {
+        for (int rg = 0; rg < n_rows; rg += 32) {
+          const T* from[8];
+#pragma unroll
+          for (int u = 0; u < 8; ++u) from[u] = src + off[min(rg + 4 * u + row_lo, n_rows - 1)] + k0 + c * 8;
+#pragma unroll
+          for (int u = 0; u < 8; ++u) {
+            const int row = rg + 4 * u + row_lo;
+            if (row < n_rows) cp_async16(dst + row * 128 + ((c ^ (row & 7)) << 4), from[u]);
+          }
+        }
+      };
       if (gather) pdl_wait();  // this warp reads the activations itself
       for (int kb = warp, use = 0; kb < nkb; kb += nst, ++use) {
         if (use > 0 && !mbar_wait_timed(&ctl.empty[warp], (use - 1) & 1)) {
@@ -398,28 +424,8 @@ __global__ void __launch_bounds__(kMmaShrinkThreads, 1)
           break;
         }
         const int k0 = (kb_base + kb) * kMmaKBlock;
-        if (gather) {
-          // token rows into the 128-byte swizzled layout the TMA would have produced: chunk c of row i at
-          // i * 128 + ((c ^ (i & 7)) << 4)
-          const uint32_t xdst = smem0 + warp * stage_bytes;
-          for (int rg = 0; rg < kMmaTokens; rg += 8) {
-            const int row = rg + row_lo;
-            const T* src = x + ctl.tok_off[row] + k0;
-#pragma unroll
-            for (int ch = 0; ch < 2; ++ch) {
-              const int c = ch * 4 + c_lo;
-              cp_async16(xdst + row * 128 + ((c ^ row_lo) << 4), src + c * 8);
-            }
-          }
-        }
-        for (int rg = 0; rg < npad; rg += 8) {
-          const T* src = w + ctl.row_off[rg + row_lo] + k0;
-#pragma unroll
-          for (int ch = 0; ch < 2; ++ch) {
-            const int c = ch * 4 + c_lo;
-            cp_async16(dst0 + c * (npad * 16) + rg * 16, src + c * 8);
-          }
-        }
+        copy_rows(w, ctl.row_off, wdst, npad, k0);
+        if (gather) copy_rows(x, ctl.tok_off, xdst, kMmaTokens, k0);
         cp_async_wait_all();
         fence_proxy_async();
         __syncwarp();
@@ -457,7 +463,7 @@ __global__ void __launch_bounds__(kMmaShrinkThreads, 1)
 #pragma unroll
         for (int ks = 0; ks < kMmaKBlock / 16; ++ks) {
           const uint64_t da = umma_smem_desc_sw128(sb + ks * 32);
-          const uint64_t db = umma_smem_desc(sb + kMmaXTileBytes + ks * 2 * (npad * 16), npad * 16, 128);
+          const uint64_t db = umma_smem_desc_sw128(sb + kMmaXTileBytes + ks * 32);
           umma_f16(tmem, da, db, idesc, (kb > 0 || ks > 0) ? 1u : 0u);
         }
         umma_commit(&ctl.empty[s]);
@@ -475,7 +481,7 @@ __global__ void __launch_bounds__(kMmaShrinkThreads, 1)
   for (int q = 0; q < gp; ++q) vec = vec && ((reinterpret_cast<uintptr_t>(pick3(a.delta, p0 + q)) & 15) == 0);
   // eight consecutive columns [j0, j0 + 8) of row `tok` (j0 a multiple of 8, so they lie in one projection)
   auto store8 = [&](int64_t tok, int j0, const float (&f)[8]) {
-    const int p = j0 / r, jj = j0 - p * r;
+    const int p = (j0 >= r ? 1 : 0) + (j0 >= 2 * r ? 1 : 0), jj = j0 - p * r;
     T* drow = reinterpret_cast<T*>(pick3(a.delta, p0 + p)) + tok * a.delta_stride;
     if (vec && jj + 8 <= a.delta_width) {
       union {
@@ -533,24 +539,42 @@ __global__ void __launch_bounds__(kMmaShrinkThreads, 1)
     // CTA kq adds the ks partial tiles for its share of the rows, in rank order, and stores them
     bool all_ok = true;
     for (int q = 0; q < ks; ++q) all_ok = all_ok && ld_peer_i32(peer_smem(smem_u32(&ctl.bad), q)) == 0;
-    if (all_ok && tid < 128) {
-      const int rows_per = kMmaTokens / ks;
-      const int groups = npad >> 3;
-      for (int u = tid; u < rows_per * groups; u += 128) {
-        const int row = kq * rows_per + u / groups;
-        const int j0 = (u % groups) * 8;
-        if (row < t.n && j0 < rows) {
+    if (all_ok) {
+      // (row, group of eight columns) pairs dealt to all threads, kept by steps; the partial tiles' values of one pair are
+      // all on their way before the first is added
+      const int rows_per = kMmaTokens / ks, groups = npad >> 3;
+      int row = tid / groups, grp = tid - row * groups;
+      const int row_step = kMmaShrinkThreads / groups, grp_step = kMmaShrinkThreads - row_step * groups;
+      while (row < rows_per) {
+        const int tile_row = kq * rows_per + row, j0 = grp * 8;
+        if (tile_row < t.n && j0 < rows) {
+          const uint32_t local = smem0 + tile_row * pitch + j0 * 4;
+          float4 part[8][2];
+#pragma unroll
+          for (int q = 0; q < 8; ++q) {
+            if (q < ks) {
+              const uint32_t pa = peer_smem(local, q);
+              part[q][0] = ld_peer_f4(pa);
+              part[q][1] = ld_peer_f4(pa + 16);
+            }
+          }
           float f[8];
 #pragma unroll
           for (int e = 0; e < 8; ++e) f[e] = 0.f;
-          const uint32_t local = smem0 + row * pitch + j0 * 4;
-          for (int q = 0; q < ks; ++q) {
-            const uint32_t pa = peer_smem(local, q);
-            const float4 lo4 = ld_peer_f4(pa), hi4 = ld_peer_f4(pa + 16);
-            f[0] += lo4.x, f[1] += lo4.y, f[2] += lo4.z, f[3] += lo4.w;
-            f[4] += hi4.x, f[5] += hi4.y, f[6] += hi4.z, f[7] += hi4.w;
+#pragma unroll
+          for (int q = 0; q < 8; ++q) {
+            if (q < ks) {
+              f[0] += part[q][0].x, f[1] += part[q][0].y, f[2] += part[q][0].z, f[3] += part[q][0].w;
+              f[4] += part[q][1].x, f[5] += part[q][1].y, f[6] += part[q][1].z, f[7] += part[q][1].w;
+            }
           }
-          store8(mma_token(t, row), j0, f);
+          store8(mma_token(t, tile_row), j0, f);
+        }
+        row += row_step;
+        grp += grp_step;
+        if (grp >= groups) {
+          grp -= groups;
+          ++row;
         }
       }
     }
@@ -613,8 +637,8 @@ __global__ void __launch_bounds__(kMmaExpandThreads)
   }
 
   // the pool rows behind outputs [o_begin, o_end) are checked before anything is copied
-  const uint32_t pr_first = static_cast<uint32_t>(o_begin) * R / S;
-  const uint32_t pr_last = (static_cast<uint32_t>(o_end) * R - 1) / S;
+  const uint32_t pr_first = a.stride.div(o_begin * R);
+  const uint32_t pr_last = a.stride.div(o_end * R - 1);
   bool rows_ok = pr_last - pr_first < sizeof(s_row_off) / sizeof(s_row_off[0]);
   for (uint32_t pr = pr_first + tid; pr <= pr_last && rows_ok; pr += kMmaExpandThreads) {
     if (pr >= static_cast<uint32_t>(R)) {
@@ -675,8 +699,6 @@ __global__ void __launch_bounds__(kMmaExpandThreads)
       const int o0 = o_begin + ch * kMmaOutChunk;
       const int ncols = min(kMmaOutChunk, o_end - o0);  // a multiple of 8
       const int npad = (ncols + 15) & ~15;
-      // the previous chunk's reduce must have finished reading the out tile
-      if (gather || tid == 0) bulk_wait_read<0>();
       const bool got = mbar_wait_timed(&ctl.acc_full[ab], (ch >> 1) & 1);
       // all four warps go on, or leave, together
       if (!named_and(128, got)) {
@@ -684,48 +706,59 @@ __global__ void __launch_bounds__(kMmaExpandThreads)
         break;
       }
       tc_fence_after();
-      const uint32_t out_tile = out_smem;
+      // 64 columns at a time: the two halves of the out tile take turns, so that the copy engine adds one while the other
+      // is written (gathered tokens: whole rows, each by the thread that wrote it)
+      if (gather) bulk_wait_read<0>();  // this thread's previous row must have been read
 #pragma unroll
-      for (int g = 0; g < kMmaOutChunk / 16; ++g) {
-        if (g * 16 < npad) {  // uniform over the warps
-          uint32_t v[16];
-          tmem_ld16(tmem + (static_cast<uint32_t>(warp * 32) << 16) + ab * kMmaOutChunk + g * 16, v);
-          tmem_ld_wait();
+      for (int half = 0; half < 2; ++half) {
+        if (half * 64 >= npad) break;  // uniform over the warps
+        if (!gather) {
+          if (tid == 0) bulk_wait_read<1>();  // what this half held before
+          named_sync(128);
+        }
 #pragma unroll
-          for (int h = 0; h < 2; ++h) {
-            union {
-              uint4 q4;
-              T e[8];
-            } pk;
+        for (int g = half * 4; g < half * 4 + 4; ++g) {
+          if (g * 16 < npad) {
+            uint32_t v[16];
+            tmem_ld16(tmem + (static_cast<uint32_t>(warp * 32) << 16) + ab * kMmaOutChunk + g * 16, v);
+            tmem_ld_wait();
 #pragma unroll
-            for (int e = 0; e < 8; ++e)
-              pk.e[e] = from_f32<T>(live ? scale * __uint_as_float(v[h * 8 + e]) : 0.f);
-            const int col = g * 16 + h * 8;  // column of the 128-wide tile; half = col / 64
-            const uint32_t cc = static_cast<uint32_t>((col & 63) >> 3);
-            const uint32_t dst =
-                gather ? out_tile + row * kMmaOutRowPitch + col * 2
-                       : out_tile + (col >> 6) * (kMmaTokens * 128) + row * 128 + ((cc ^ (row & 7)) << 4);
-            asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(dst), "r"(pk.q4.x), "r"(pk.q4.y),
-                         "r"(pk.q4.z), "r"(pk.q4.w)
-                         : "memory");
+            for (int h = 0; h < 2; ++h) {
+              union {
+                uint4 q4;
+                T e[8];
+              } pk;
+#pragma unroll
+              for (int e = 0; e < 8; ++e)
+                pk.e[e] = from_f32<T>(live ? scale * __uint_as_float(v[h * 8 + e]) : 0.f);
+              const int col = g * 16 + h * 8;  // column of the 128-wide tile
+              const uint32_t cc = static_cast<uint32_t>((col & 63) >> 3);
+              const uint32_t dst =
+                  gather ? out_smem + row * kMmaOutRowPitch + col * 2
+                         : out_smem + half * (kMmaTokens * 128) + row * 128 + ((cc ^ (row & 7)) << 4);
+              asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(dst), "r"(pk.q4.x), "r"(pk.q4.y),
+                           "r"(pk.q4.z), "r"(pk.q4.w)
+                           : "memory");
+            }
+          }
+        }
+        if (!gather) {
+          fence_proxy_async();
+          named_sync(128);
+          if (tid == 0) {
+            tma_reduce_add_2d(ymap, o0 + half * 64, t.first, out_smem + half * (kMmaTokens * 128));
+            bulk_commit();
           }
         }
       }
       tc_fence_before();
       __syncwarp();
       if (lane == 0) mbar_arrive(&ctl.acc_empty[ab]);
-      fence_proxy_async();
       if (gather) {
         // each thread adds the row it wrote itself: no barrier needed
-        if (live) bulk_reduce_add<T>(yrow + o0, out_tile + row * kMmaOutRowPitch, static_cast<uint32_t>(ncols) * 2);
+        fence_proxy_async();
+        if (live) bulk_reduce_add<T>(yrow + o0, out_smem + row * kMmaOutRowPitch, static_cast<uint32_t>(ncols) * 2);
         bulk_commit();
-      } else {
-        named_sync(128);
-        if (tid == 0) {
-          for (int half = 0; half * 64 < ncols; ++half)
-            tma_reduce_add_2d(ymap, o0 + half * 64, t.first, out_tile + half * (kMmaTokens * 128));
-          bulk_commit();
-        }
       }
     }
     if (gather || tid == 0) bulk_wait<0>();
@@ -734,6 +767,20 @@ __global__ void __launch_bounds__(kMmaExpandThreads)
     const int lw = warp - 4;
     const T* wsrc = reinterpret_cast<const T*>(a.w);
     const int n_items = kMmaTokens * cpr;
+    // 16-byte piece q of a tile is piece c of row `row`: kept by steps, for a division costs more than the copy (with two
+    // of them a piece this loop, not memory, set the kernel's time)
+    const int row0 = lane / cpr, c0 = lane - row0 * cpr;
+    const int row32 = 32 / cpr, c32 = 32 - row32 * cpr;
+    auto step = [&](int& row, int& c, int by) {
+      for (int k = 0; k < by; k += 32) {
+        row += row32;
+        c += c32;
+        if (c >= cpr) {
+          c -= cpr;
+          ++row;
+        }
+      }
+    };
     if (kpad != R) {
       // the chunk that pads K to a multiple of 16 is zero in all operand tiles and never overwritten
       for (int i = lw * 32 + lane; i < 3 * kMmaTokens; i += kMmaExLoaderWarps * 32) {
@@ -752,20 +799,24 @@ __global__ void __launch_bounds__(kMmaExpandThreads)
         }
         const int o0 = o_begin + ch * kMmaOutChunk;
         const uint32_t dst = b_smem + s * tile_bytes;
+        int row = row0, c = c0;
+#pragma unroll 4
         for (int q = lane; q < n_items; q += 32) {
-          const int row = q / cpr, c = q - row * cpr;
-          const uint32_t o = static_cast<uint32_t>(min(o0 + row, h_out - 1));
-          const uint32_t f = o * R + c * 8;
-          const uint32_t pr = f / S, col = f - pr * S;
+          const int f = min(o0 + row, h_out - 1) * R + c * 8;
+          const uint32_t pr = a.stride.div(f), col = f - pr * S;
           cp_async16(dst + c * kLbo + row * 16, wsrc + s_row_off[pr - pr_first] + col);
+          step(row, c, 32);
         }
       }
       if (first) {
         pdl_wait();  // delta comes from the kernel before this one
         const T* dsrc = reinterpret_cast<const T*>(pick3(a.delta, p));
+        int row = row0, c = c0;
+        if (lw > 0) step(row, c, lw * 32);
+#pragma unroll 4
         for (int q = lw * 32 + lane; q < n_items; q += kMmaExLoaderWarps * 32) {
-          const int row = q / cpr, c = q - row * cpr;
           cp_async16(d_smem + c * kLbo + row * 16, dsrc + mma_token(t, row) * a.delta_stride + c * 8);
+          step(row, c, kMmaExLoaderWarps * 32);
         }
       }
       cp_async_wait_all();

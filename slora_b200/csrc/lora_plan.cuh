@@ -24,7 +24,11 @@ __global__ void __launch_bounds__(1024) plan_build_kernel(int32_t* ws, const int
   int32_t* cnt = pos + T;
   const int big_off = (PH_WORDS + kTileWords * max_tiles + 2 * T + n_adapters + 3) & ~3;  // 16-byte aligned records
   int32_t* big = ws + big_off;
-  __shared__ int s_tok[32], s_tile[32], s_big[32];
+  // big groups keep the batch's token order (a prompt's tokens then lie in consecutive slots, and the tensor-core kernels
+  // can move whole tiles).  Until perm is filled, a group's first slot in it holds its number among the big groups, -1
+  // for the others.
+  __shared__ int s_seen[32][kOrderedGroups];
+  __shared__ int s_tok[32], s_tile[32], s_big[32], s_ngroups;
   __shared__ int s_status, s_rmin, s_rmax, s_nsmall, s_big_rmax, s_big_pow2;
   const int tid = threadIdx.x, nthr = blockDim.x, lane = tid & 31, warp = tid >> 5;
 
@@ -36,7 +40,9 @@ __global__ void __launch_bounds__(1024) plan_build_kernel(int32_t* ws, const int
     s_nsmall = 0;
     s_big_rmax = 0;
     s_big_pow2 = 1;
+    s_ngroups = 0;
   }
+  for (int i = tid; i < 32 * kOrderedGroups; i += nthr) s_seen[i / kOrderedGroups][i % kOrderedGroups] = 0;
   __syncthreads();
   for (int t = tid; t < T; t += nthr) {
     const int64_t a = ids[t];
@@ -112,6 +118,7 @@ __global__ void __launch_bounds__(1024) plan_build_kernel(int32_t* ws, const int
   for (int a = lo; a < hi; ++a) {
     const int c = cnt[a];
     cnt[a] = tok_off;  // becomes the group's first slot in perm
+    int group = -1;
     if (c > 0) {
       const int64_t r4 = ranks4[a], st = start[a];
       const bool good = r4 >= 0 && st >= 0 && st + r4 <= loc_len && r4 <= (int64_t(1) << 20) && st < 0x7fffffffLL;
@@ -125,6 +132,8 @@ __global__ void __launch_bounds__(1024) plan_build_kernel(int32_t* ws, const int
         const int rr = static_cast<int>(r4 >> 2);
         atomicMax(&s_big_rmax, rr);
         if (rr & (rr - 1)) s_big_pow2 = 0;
+        const int g = atomicAdd(&s_ngroups, 1);
+        if (g < kOrderedGroups) group = g;
       } else if (good) {
         atomicAdd(&s_nsmall, (c + kTileTokens - 1) / kTileTokens);
       }
@@ -143,18 +152,63 @@ __global__ void __launch_bounds__(1024) plan_build_kernel(int32_t* ws, const int
             int4* rec = reinterpret_cast<int4*>(big + kTileWords * bigt_off);
             rec[0] = make_int4(a, tok_off + i * kBigTileTokens, min(kBigTileTokens, c - i * kBigTileTokens),
                                static_cast<int>(r4 >> 2));
-            rec[1] = make_int4(static_cast<int>(st), 0, 0, 0);
+            rec[1] = make_int4(static_cast<int>(st), 0, 0, group >= 0 ? 1 : 0);
           }
           ++bigt_off;
         }
       }
     }
+    if (c > 0) perm[tok_off] = group;
     tok_off += c;
   }
   __syncthreads();
+  if (s_ngroups > 0) {
+    // each warp owns a run of the batch: it counts the big groups' tokens in it, the warps' counts become starts, and a
+    // second walk in order numbers the tokens
+    const int nw = nthr >> 5, run = ((T + nw - 1) / nw + 31) & ~31;
+    const int t0 = min(warp * run, T), t1 = min(t0 + run, T);
+    for (int walk = 0; walk < 2; ++walk) {
+      for (int tb = t0; tb < t1; tb += 32) {
+        const int t = tb + lane;
+        int g = -1;
+        if (t < t1) {
+          const int64_t a = ids[t];
+          if (a >= 0 && a < n_adapters) g = perm[cnt[a]];
+        }
+        const uint32_t same = __match_any_sync(0xffffffffu, g);
+        if (g >= 0) {
+          if (walk == 1) pos[t] = s_seen[warp][g] + __popc(same & ((1u << lane) - 1));
+        }
+        __syncwarp();
+        if (g >= 0 && lane == __ffs(same) - 1) s_seen[warp][g] += __popc(same);
+        __syncwarp();
+      }
+      __syncthreads();
+      if (walk == 0) {
+        if (tid < kOrderedGroups) {
+          int sum = 0;
+          for (int w = 0; w < nw; ++w) {
+            const int v = s_seen[w][tid];
+            s_seen[w][tid] = sum;
+            sum += v;
+          }
+        }
+        __syncthreads();
+      }
+    }
+  }
   for (int t = tid; t < T; t += nthr) {
     const int p = pos[t];
     if (p >= 0) perm[cnt[ids[t]] + p] = t;
+  }
+  __syncthreads();
+  // big tiles whose tokens are consecutive (sorted: the first and the last tell)
+  for (int i = tid; i < hdr[PH_NBIG]; i += nthr) {
+    int32_t* rec = big + kTileWords * i;
+    const int first = rec[1], n = rec[2];
+    const int lo = perm[first], hi = perm[first + n - 1];
+    rec[5] = rec[7] != 0 && hi - lo == n - 1 ? 1 : 0;
+    rec[6] = lo;
   }
   // resolved tiles (see PH_XOFF): token ids, scale and pool rows of every tile whose rank the entries hold
   if (xoff > 0 && loc != nullptr) {
