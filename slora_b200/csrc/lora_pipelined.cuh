@@ -98,7 +98,6 @@ struct PipeCtl {
   uint64_t full[kSlots];
   uint64_t empty[kSlots];
   int meta[kSlots][16];
-  uint32_t off[kProducerWarps][kSlots];  // byte offset of each stage in the ring (a copy per producer warp)
   // the 32 items a batch resolves, one per lane of the first producer warp, parked here for the lanes that carry the
   // copies: pool rows and the item's description
   int32_t d_l[32][kItemRows];
@@ -118,12 +117,13 @@ struct ShrinkRed {
   int cnt[kSlots];
 };
 
-// Producer-side ring state (identical in all 32 lanes).
+// Producer-side ring state (identical in all 32 lanes, but for `off`).
 struct Ring {
   int role = 0;       // which producer warp this is
   uint32_t g = 0;     // next stage index
   uint32_t tail = 0;  // oldest stage not yet known to be released
   uint32_t head = 0;  // next free byte
+  uint32_t off = 0;   // lane s: byte offset of the stage in slot s
   bool pre = true;    // still before the grid-dependency wait
   bool dead = false;  // a bounded wait ran out
   uint32_t cap = kRingBytes;  // bytes of the ring
@@ -258,7 +258,9 @@ __device__ __forceinline__ void ring_enter(Ring& r, int lane) {
 }
 
 // Reserve `sz` bytes (a multiple of 128) and a descriptor for stage r.g; returns the byte offset, or 0xffffffff when
-// a wait ran out.
+// a wait ran out.  The lanes poll the barriers one by one, so every turn of the loop brings them together again: each
+// issues copies of its own, and a lane that saw another stage's offset would send its copy into a stage in use.  What
+// they share of earlier stages therefore goes through shuffles and votes, not through shared memory.
 __device__ __forceinline__ uint32_t ring_alloc(Ring& r, PipeCtl& c, uint32_t sz, int lane) {
   for (;;) {
     uint32_t cand = 0;
@@ -267,7 +269,7 @@ __device__ __forceinline__ uint32_t ring_alloc(Ring& r, PipeCtl& c, uint32_t sz,
       r.head = 0;
       ok = true;
     } else {
-      const uint32_t t = c.off[r.role][r.tail % kSlots];
+      const uint32_t t = __shfl_sync(FULL_MASK, r.off, r.tail % kSlots);
       if (r.head > t) {
         if (r.head + sz <= r.cap) {
           cand = r.head;
@@ -281,9 +283,13 @@ __device__ __forceinline__ uint32_t ring_alloc(Ring& r, PipeCtl& c, uint32_t sz,
         ok = r.head + sz <= t && r.head != t;
       }
     }
-    if (ok && r.g - r.tail < r.slots) return cand;
+    if (ok && r.g - r.tail < r.slots) {
+      r.head = cand + sz;
+      if (lane == static_cast<int>(r.g % kSlots)) r.off = cand;
+      return cand;
+    }
     ring_enter(r, lane);
-    if (!mbar_wait_timed(&c.empty[r.tail % kSlots], (r.tail / kSlots) & 1)) {
+    if (!__all_sync(FULL_MASK, mbar_wait_timed(&c.empty[r.tail % kSlots], (r.tail / kSlots) & 1))) {
       r.dead = true;
       return 0xffffffffu;
     }
@@ -308,6 +314,7 @@ __device__ __forceinline__ void ring_issue(Ring& r, PipeCtl& c, uint32_t slot, u
 
 // The producer warps meet: before a batch of items is resolved (all of them are done with the previous one) and after.
 __device__ __forceinline__ void producers_sync() {
+  __syncwarp();  // (a barrier of whole warps)
   asm volatile("bar.sync 1, %0;" ::"n"(kProducerWarps * 32) : "memory");
 }
 
@@ -678,8 +685,6 @@ __device__ __forceinline__ void shrink_producer(const ShrinkArgs& a, unsigned ch
         const uint32_t off = ring_alloc(r, c, sz, lane);
         if (r.dead) break;
         const uint32_t slot = r.g % kSlots;
-        r.head = off + sz;
-        if (lane == 0) c.off[role][slot] = off;
         if (role == 0) {
           if (lane == 0) {  // the stage record in two 16-byte stores; [7] = slot rows of the adapter
             int4* mrec = reinterpret_cast<int4*>(c.meta[slot]);
@@ -1152,8 +1157,6 @@ __device__ __forceinline__ void expand_producer(const ExpandArgs& a, unsigned ch
       const uint32_t off = ring_alloc(r, c, sz, lane);
       if (r.dead) break;
       const uint32_t slot = r.g % kSlots;
-      r.head = off + sz;
-      if (lane == 0) c.off[role][slot] = off;
       if (role == 0) {
         if (lane == 0) {  // the stage record in two 16-byte stores
           int4* mrec = reinterpret_cast<int4*>(c.meta[slot]);
