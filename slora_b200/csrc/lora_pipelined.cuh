@@ -111,7 +111,7 @@ struct PipeCtl {
 // Shrink only: per-item partial sums of the consumer warps and the arrival counter that elects the last warp.  (Kept
 // out of PipeCtl so that the expand, which has no use for it, can give those 8 KB to its ring.)
 // Rows of a C fragment: half h holds rows 8h + lane / 4, tokens 2 (lane % 4) and the next; four, eight or sixteen rows
-// are a half fragment (the lanes below 16), one or two.  8 KB hold the items that shrink_slots() lets be in flight.
+// are a half fragment (the lanes below 16), one or two.  8 KB hold the shrink_buffers() of a launch.
 struct ShrinkRed {
   float2 sum[4 * kConsumerWarps * 32];
   int cnt[kSlots];
@@ -257,33 +257,32 @@ __device__ __forceinline__ void ring_enter(Ring& r, int lane) {
   }
 }
 
-// Reserve `sz` bytes (a multiple of 128) and a descriptor for stage r.g; returns the byte offset, or 0xffffffff when
-// a wait ran out.  The lanes poll the barriers one by one, so every turn of the loop brings them together again: each
-// issues copies of its own, and a lane that saw another stage's offset would send its copy into a stage in use.  What
-// they share of earlier stages therefore goes through shuffles and votes, not through shared memory.
-__device__ __forceinline__ uint32_t ring_alloc(Ring& r, PipeCtl& c, uint32_t sz, int lane) {
+// Where `sz` bytes go in a ring of `cap` bytes whose next free byte is `head` and whose oldest stage in use starts at
+// `oldest` (`empty`: none is in use).
+__host__ __device__ __forceinline__ bool ring_fits(uint32_t head, bool empty, uint32_t oldest, uint32_t cap, uint32_t sz,
+                                                   uint32_t& at) {
+  at = 0;
+  if (empty) return true;
+  if (head <= oldest) {  // wrapped
+    at = head;
+    return head + sz <= oldest && head != oldest;
+  }
+  if (head + sz > cap) return sz <= oldest;
+  at = head;
+  return true;
+}
+
+// Reserve `sz` bytes (a multiple of 128) and a descriptor for stage r.g, once all stages before `released` have been
+// released; returns the byte offset, or 0xffffffff when a wait ran out.  The lanes poll the barriers one by one, so every
+// turn of the loop brings them together again: each issues copies of its own, and a lane that saw another stage's offset
+// would send its copy into a stage in use.  What they share of earlier stages therefore goes through shuffles and votes,
+// not through shared memory.
+__device__ __forceinline__ uint32_t ring_alloc(Ring& r, PipeCtl& c, uint32_t sz, int lane, uint32_t released = 0) {
   for (;;) {
-    uint32_t cand = 0;
-    bool ok;
-    if (r.tail == r.g) {
-      r.head = 0;
-      ok = true;
-    } else {
-      const uint32_t t = __shfl_sync(FULL_MASK, r.off, r.tail % kSlots);
-      if (r.head > t) {
-        if (r.head + sz <= r.cap) {
-          cand = r.head;
-          ok = true;
-        } else {
-          cand = 0;
-          ok = sz <= t;
-        }
-      } else {
-        cand = r.head;
-        ok = r.head + sz <= t && r.head != t;
-      }
-    }
-    if (ok && r.g - r.tail < r.slots) {
+    uint32_t cand;
+    const uint32_t oldest = __shfl_sync(FULL_MASK, r.off, r.tail % kSlots);
+    const bool ok = ring_fits(r.head, r.tail == r.g, oldest, r.cap, sz, cand);
+    if (ok && r.g - r.tail < r.slots && static_cast<int32_t>(r.tail - released) >= 0) {
       r.head = cand + sz;
       if (lane == static_cast<int>(r.g % kSlots)) r.off = cand;
       return cand;
@@ -352,7 +351,7 @@ __device__ __forceinline__ P pick3(P const (&arr)[3], int p) {
   return p == 0 ? arr[0] : (p == 1 ? arr[1] : arr[2]);
 }
 
-__device__ __forceinline__ uint32_t round128(uint32_t v) { return (v + 127u) & ~127u; }
+__host__ __device__ __forceinline__ uint32_t round128(uint32_t v) { return (v + 127u) & ~127u; }
 
 // ------------------------------------------------------------------------------------------------------------
 // Which items does a launch have?  A tile yields a number of items that depends on its adapter's rank (row blocks
@@ -517,7 +516,7 @@ __device__ __forceinline__ int proj_of(int rem, int nb, int nproj) {
 // Chunk j of a stage starts (j + 1) / 2 * kChunkPad bytes after j chunks' values: two rows that lie next to each other
 // start in different halves of the banks, so that the eight lanes that read 64 bytes of each do not collide.
 constexpr int kChunkPad = 64;
-__device__ __forceinline__ int chunk_at(int j, int bytes) { return j * bytes + ((j + 1) >> 1) * kChunkPad; }
+__host__ __device__ __forceinline__ int chunk_at(int j, int bytes) { return j * bytes + ((j + 1) >> 1) * kChunkPad; }
 // K elements of a shrink stage of `chunks` rows and tokens, in pairs of units of kKUnit: what fits kMaxStageBytes, at
 // least one pair.
 constexpr int kKUnit = 512;
@@ -535,17 +534,34 @@ constexpr StagePairs stage_pairs_table() {
 }
 constexpr uint64_t kPairs0 = stage_pairs_table().w[0], kPairs1 = stage_pairs_table().w[1],
                    kPairs2 = stage_pairs_table().w[2];
-__device__ __forceinline__ int stage_k(int chunks) {
+__host__ __device__ __forceinline__ int stage_k(int chunks) {
   const int i = chunks - 1;
   const uint64_t w = i < 8 ? kPairs0 : (i < 16 ? kPairs1 : kPairs2);
   return static_cast<int>((w >> (8 * (i & 7))) & 255u) * (2 * kKUnit);
 }
-// Reduction buffers (items in flight) and stages in flight of a launch.  Stages in flight touch at most one item more
-// than the whole items among them: three stages of items of two or more are two items.
-__device__ __forceinline__ uint32_t shrink_buffers(int rows_per_item) { return rows_per_item > 8 ? 2 : (rows_per_item > 4 ? 4 : 8); }
-__device__ __forceinline__ uint32_t shrink_slots(int rows_per_item, int h_in) {
-  return rows_per_item > 8 ? (h_in > stage_k(kItemRows + 1) ? 3 : 2) : shrink_buffers(rows_per_item);
+// Reduction buffers of a launch: items whose last stage may be in flight at once.  Item i sums in buffer i mod
+// buffers, so its last stage goes out only when item i - buffers has been released.  Up to eight rows there are as many
+// buffers as stages may be in flight, which is all it takes.  Items of sixteen rows have two (4 KB each): how many stages
+// an item has depends on its rows and tokens (eight rows and a token are one up to 2048 elements, two rows up to 8192),
+// so the producers count items and not stages, and the ring's bytes bound the stages.
+__host__ __device__ __forceinline__ uint32_t shrink_buffers(int rows_per_item) {
+  return rows_per_item > 8 ? 2 : (rows_per_item > 4 ? 4 : 8);
 }
+__host__ __device__ __forceinline__ uint32_t shrink_slots(int rows_per_item) {
+  return rows_per_item > 8 ? kSlots : shrink_buffers(rows_per_item);
+}
+// The ends of the two items before the current one, as the number of stages up to there.
+struct ItemEnds {
+  uint32_t previous = 0, before = 0;
+  // The stages that have to be released before the next one goes out.
+  __host__ __device__ __forceinline__ uint32_t released(bool item_ends, int rows_per_item) const {
+    return item_ends && rows_per_item > 8 ? before : 0;
+  }
+  __host__ __device__ __forceinline__ void end_item(uint32_t stages) {
+    before = previous;
+    previous = stages;
+  }
+};
 
 template <typename T, bool EXACT>
 __device__ __forceinline__ void shrink_producer(const ShrinkArgs& a, unsigned char* ring_mem, PipeCtl& c, int lane,
@@ -560,7 +576,8 @@ __device__ __forceinline__ void shrink_producer(const ShrinkArgs& a, unsigned ch
   Ring r;
   r.role = role;
   r.cap = kShrinkRingBytes;
-  r.slots = shrink_slots(RB, h_in);
+  r.slots = shrink_slots(RB);
+  ItemEnds ends;
   r.trigger_after_wait = a.tp.enabled && a.tp.inband >= 2;
   const ItemMap map = EXACT ? build_item_map(a.src, a.nproj * a.max_rb, c, lane, role,
                                              [&](int rr, int) { return shrink_items_of(a, rr); })
@@ -682,13 +699,14 @@ __device__ __forceinline__ void shrink_producer(const ShrinkArgs& a, unsigned ch
         const int klen = min(kc_elems, h_in - k0);
         const uint32_t bytes = static_cast<uint32_t>(klen) * sizeof(T);
         const uint32_t sz = round128(chunk_at(nrows + n, bytes));
-        const uint32_t off = ring_alloc(r, c, sz, lane);
+        const bool last = k0 + klen >= h_in;
+        const uint32_t off = ring_alloc(r, c, sz, lane, ends.released(last, RB));
         if (r.dead) break;
         const uint32_t slot = r.g % kSlots;
         if (role == 0) {
           if (lane == 0) {  // the stage record in two 16-byte stores; [7] = slot rows of the adapter
             int4* mrec = reinterpret_cast<int4*>(c.meta[slot]);
-            mrec[0] = make_int4((k0 == 0 ? FLAG_FIRST : 0) | (k0 + klen >= h_in ? FLAG_LAST : 0), nrows, n, m_j0);
+            mrec[0] = make_int4((k0 == 0 ? FLAG_FIRST : 0) | (last ? FLAG_LAST : 0), nrows, n, m_j0);
             mrec[1] = make_int4(m_p, klen, static_cast<int>(off), m_rows);
           } else if (lane >= kActLane && lane < kActLane + kTileTokens) {
             c.meta[slot][8 + lane - kActLane] = mytok;
@@ -702,6 +720,7 @@ __device__ __forceinline__ void shrink_producer(const ShrinkArgs& a, unsigned ch
                                     : is_x || (is_w && r.g >= kRowsAhead && lane >= (nrows + n + 1) / 2);
         ring_issue(r, c, slot, ring_base + off + chunk_at(myslot, bytes), src0 + k0,
                    mine ? bytes : 0u);
+        if (last) ends.end_item(r.g);
       }
     }
     __syncwarp();
@@ -808,8 +827,8 @@ __device__ __forceinline__ void shrink_partials(const ShrinkAcc& acc, float (&ou
 }
 
 // At the item's last chunk the warps' partial sums meet in shared memory; the warp that arrives last (an atomic counter,
-// no waiting) adds them in a fixed order and writes delta.  A reduction buffer is reused only as many items later as the
-// ring may hold stages, which is after the last warp released the stage it was summing in.
+// no waiting) adds them in a fixed order and writes delta.  A reduction buffer is reused only after the last warp released
+// the stage it was summing in (shrink_buffers).
 template <typename T, bool EXACT>
 __device__ __forceinline__ void shrink_consumer(const ShrinkArgs& a, const unsigned char* ring_mem, PipeCtl& c,
                                                 ShrinkRed& red, int lane, int cw) {

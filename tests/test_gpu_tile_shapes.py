@@ -91,3 +91,35 @@ def test_ranks_that_fill_no_block():
         for t, a in enumerate(wl.ids.tolist()):
             r = wl.ranks[a]
             np.testing.assert_allclose(got[t, :r], ref[t, :r], rtol=2e-3, atol=2e-3)
+
+
+def _few_at_a_time(wl, n=48):
+    """Per-token calls of `n` tokens: too few items for more than four rows each."""
+    w = wl.to(DEV)
+    ops = sl.LoraBatchOps(w.a_start, w.a_len, w.a_loc, w.a_scaling, w.pools_a, w.pools_b, wl.max_rank)
+    outs = [torch.zeros((wl.T, ho), dtype=wl.dtype, device=DEV) for _, ho in wl.proj_dims()]
+    for at in range(0, wl.T, n):
+        part = slice(at, at + n)
+        ops.prepare(w.ids[part], use_plan=False)
+        ops.lora_get_qkv(0, w.x_qkv[0][part], *(o[part] for o in outs[:3]))
+        ops.lora_get_o(0, w.x_o[0][part], outs[3][part])
+    torch.cuda.synchronize()
+    return outs
+
+
+@pytest.mark.parametrize("exact", [False, True])
+@pytest.mark.parametrize("hidden", [640, 1280, 1536, 2048])
+def test_partly_filled_items_of_sixteen_rows(hidden, exact):
+    """Ranks of 8 and 64 in items of sixteen rows, tiles of one token and of many: at these hidden sizes a short item is one
+    stage and a long one several, and the launch has two reduction buffers (tests/ring_model.cu)."""
+    wl = build_workload(5, pool_rows=200 * 4 * 64, n_adapters=200, decode_tokens=2048, hidden=hidden, h_kv=hidden,
+                        rank_choices=(8, 64))
+    # half of the adapters have one token, the others share the rest
+    wl.ids = torch.cat([torch.arange(100), 100 + torch.arange(1948) % 100])
+    single, ref = _few_at_a_time(wl), _oracle(wl)
+    for turn in range(3):
+        planned = _layer(wl, mixed_ranks=exact, big_groups=False)
+        for p in range(4):
+            assert torch.equal(planned[p], single[p]), (turn, p)
+    for p in range(4):
+        assert_parity(planned[p], ref[p], what=f"H={hidden} proj {p}")
