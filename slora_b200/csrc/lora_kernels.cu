@@ -822,8 +822,10 @@ int run_expand(const TileSrc& src, const Tables& tb, const void* w, const void* 
     const int64_t grid = mma_tiles * m.chunk_begin[nproj];
     TmapSet y_maps;
     memset(&y_maps, 0, sizeof(y_maps));
-    for (int p = 0; p < nproj && !rc; ++p)
+    for (int p = 0; p < nproj && !rc; ++p) {
       rc = make_tmap(&y_maps.m[p], dtype, y[p], h_out[p], src.T, y_stride[p], kMmaTokens);
+      if (!rc) rc = make_tmap(&y_maps.m8[p], dtype, y[p], h_out[p], src.T, y_stride[p], 8);
+    }
     if (rc) return rc;
     // (calls chained with programmatic dependent launch stay on one stream: measured, the chain's overlap is worth
     // more than running the pair side by side)

@@ -12,8 +12,9 @@
 //            tcgen05.commit, four warps read the accumulator back with tcgen05.ld and store delta.
 //   expand   two loader warps gather chunks of 128 outputs of B with cp.async, one lane issues the MMAs into a
 //            double-buffered accumulator, four warps scale and round the result into a swizzled shared-memory tile
-//            that one lane adds into y with a TMA reduce (an element-wise 16-bit add in L2, which is also how the
-//            reference accumulates: it rounds the FP32 sum to the output type and then adds, bgmv_impl.cuh:185-199).
+//            that the copy engine adds into y (TMA reduces, an element-wise 16-bit add in L2, which is also how the
+//            reference accumulates: it rounds the FP32 sum to the output type and then adds, bgmv_impl.cuh:185-199;
+//            by eight rows, and row by row what does not fill eight and where a tile's tokens lie apart).
 //
 // What bounds them (measured on B200, clock64 in every phase): the loaders' instructions.  A 16-byte cp.async that
 // touches 8 rows x 64 bytes, with the row offset read from shared memory between two copies, took 280 cycles a warp
@@ -60,7 +61,8 @@ constexpr int kMmaExpandCols = 256;                              // two accumula
 
 // Tensor maps of the y buffers of one expand call.
 struct TmapSet {
-  CUtensorMap m[3];
+  CUtensorMap m[3];   // boxes of 128 rows: full tiles
+  CUtensorMap m8[3];  // of 8 rows: tiles of fewer tokens
 };
 
 // ---- PTX wrappers ---------------------------------------------------------------------------------------------
@@ -685,13 +687,20 @@ __global__ void __launch_bounds__(kMmaExpandThreads)
   const uint32_t tmem = ctl.tmem;
 
   if (warp < 4) {
-    // ---- epilogue: scale, round, stage in shared memory, add into y with a TMA reduce (consecutive tokens: one
-    // tile reduce per 64 columns; gathered tokens: one bulk reduce per token row, issued by the row's own thread) ----
+    // ---- epilogue: scale, round, stage in shared memory, add into y with the copy engine (consecutive tokens: one tile
+    // reduce per 64 columns, or one for every eight rows where the tile is not full; gathered tokens: one bulk reduce
+    // per token row, issued by the row's own thread) ----
     const float scale = to_f32<T>(reinterpret_cast<const T*>(a.scales)[t.adapter]);
     const int row = warp * 32 + lane;
     const bool live = row < t.n;
     const bool gather = t.perm != nullptr;
-    const CUtensorMap* ymap = &y_maps.m[p];
+    // A tile reduce touches all of its rows.  Rows that are not this tile's belong to other tokens, which the tile kernel of
+    // the same call may be updating at that moment, or to nobody (an id without an adapter); rows past the batch do not
+    // count, the tensor map leaves them out.  So a tile that is not full is added by eights and its last tokens one by one.
+    const bool full = !gather && (t.n == kMmaTokens || t.first + t.n >= a.src.T);
+    const int eights = t.n & ~7;
+    const bool single = !gather && !full && live && row >= eights;
+    const CUtensorMap *ymap = &y_maps.m[p], *ymap8 = &y_maps.m8[p];
     T* yrow = reinterpret_cast<T*>(pick3(a.y, p)) + mma_token(t, live ? row : 0) * pick3(a.y_stride, p);
     pdl_wait();  // y is also written by the kernel before this one
     for (int ch = 0; ch < nch; ++ch) {
@@ -707,14 +716,18 @@ __global__ void __launch_bounds__(kMmaExpandThreads)
       }
       tc_fence_after();
       // 64 columns at a time: the two halves of the out tile take turns, so that the copy engine adds one while the other
-      // is written (gathered tokens: whole rows, each by the thread that wrote it)
+      // is written (gathered tokens: whole rows).  In a tile that is not full a warp adds its own 32 rows.
       if (gather) bulk_wait_read<0>();  // this thread's previous row must have been read
 #pragma unroll
       for (int half = 0; half < 2; ++half) {
         if (half * 64 >= npad) break;  // uniform over the warps
         if (!gather) {
-          if (tid == 0) bulk_wait_read<1>();  // what this half held before
-          named_sync(128);
+          bulk_wait_read<1>();  // what this half held before
+          if (full) {
+            named_sync(128);
+          } else {
+            __syncwarp();
+          }
         }
 #pragma unroll
         for (int g = half * 4; g < half * 4 + 4; ++g) {
@@ -735,7 +748,7 @@ __global__ void __launch_bounds__(kMmaExpandThreads)
               const uint32_t cc = static_cast<uint32_t>((col & 63) >> 3);
               const uint32_t dst =
                   gather ? out_smem + row * kMmaOutRowPitch + col * 2
-                         : out_smem + half * (kMmaTokens * 128) + row * 128 + ((cc ^ (row & 7)) << 4);
+                         : out_smem + half * (kMmaTokens * 128) + row * 128 + ((single ? cc : cc ^ (row & 7)) << 4);
               asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(dst), "r"(pk.q4.x), "r"(pk.q4.y),
                            "r"(pk.q4.z), "r"(pk.q4.w)
                            : "memory");
@@ -743,12 +756,20 @@ __global__ void __launch_bounds__(kMmaExpandThreads)
           }
         }
         if (!gather) {
+          const uint32_t out_half = out_smem + half * (kMmaTokens * 128);
           fence_proxy_async();
-          named_sync(128);
-          if (tid == 0) {
-            tma_reduce_add_2d(ymap, o0 + half * 64, t.first, out_smem + half * (kMmaTokens * 128));
-            bulk_commit();
+          if (full) {
+            named_sync(128);
+            if (tid == 0) tma_reduce_add_2d(ymap, o0 + half * 64, t.first, out_half);
+          } else {
+            __syncwarp();
+            const int box = warp * 32 + lane * 8;
+            if (lane < 4 && box < eights) tma_reduce_add_2d(ymap8, o0 + half * 64, t.first + box, out_half + box * 128);
+            if (single)
+              bulk_reduce_add<T>(yrow + o0 + half * 64, out_half + row * 128,
+                                 static_cast<uint32_t>(min(64, ncols - half * 64)) * 2);
           }
+          bulk_commit();
         }
       }
       tc_fence_before();
@@ -761,7 +782,7 @@ __global__ void __launch_bounds__(kMmaExpandThreads)
         bulk_commit();
       }
     }
-    if (gather || tid == 0) bulk_wait<0>();
+    bulk_wait<0>();
   } else if (warp < 4 + kMmaExLoaderWarps) {
     // ---- loader warps: the delta tile once, then B chunks lw, lw + 2, ... ----
     const int lw = warp - 4;
