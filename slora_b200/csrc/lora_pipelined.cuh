@@ -730,11 +730,12 @@ __device__ __forceinline__ void shrink_producer(const ShrinkArgs& a, unsigned ch
 }
 
 // Sums of one warp over its slices of an item.  K goes by units of kKUnit elements; warp cw owns [cw * 64, +64) of each, two
-// fragments of 32.  Four sums are kept apart (unit odd or even, first or second fragment), four short chains of mma
-// instead of one long one, and added in one order at the end.  The two of a unit's fragments may share one instruction:
-// where rows and tokens leave half of it empty (SPLIT), the second fragment's rows and tokens take those places.
+// fragments of 32.  A fragment of a unit is a chain of two mma from zero, added to the fragment's sum in unit order: an mma
+// truncates what it adds to its accumulator, and with accumulators kept over the whole row (sixteen steps at 8192) 1.6 of a
+// thousand intermediates were not the nearest 16-bit value, 0.9 with FMA sums.  The two fragments may share one
+// instruction: where rows and tokens leave half of it empty (SPLIT), the second fragment's rows and tokens take those places.
 struct ShrinkAcc {
-  float d[2][2][4];  // [unit parity][fragment; 0 alone when they share][C fragment]
+  float d[2][4];  // [fragment; 0 alone when they share][C fragment]
 };
 enum ShrinkForm {
   FORM_FULL,   // rows 0..7 and 8..15, tokens 0..7
@@ -749,7 +750,7 @@ __device__ __forceinline__ int shrink_form(int rows_per_item, int nrows, int n) 
 }
 
 // Lane (g, t) reads 16-byte vector t of the 64 bytes of a row or token; rows and tokens beyond the real counts, and what
-// lies beyond the rows' end (rows end anywhere on a multiple of eight elements), are zero.  A stage starts at an even
+// lies beyond the rows' end (rows end anywhere on a multiple of eight elements), are zero.  A stage starts at a whole
 // unit.  The loads of a round are issued before its first mma: the warp has nothing else to hide their latency with.
 template <typename T, int FORM>
 __device__ __forceinline__ void shrink_accumulate(ShrinkAcc& acc, const unsigned char* st, int nrows, int n, int klen,
@@ -785,23 +786,21 @@ __device__ __forceinline__ void shrink_accumulate(ShrinkAcc& acc, const unsigned
     pa += 2 * UNITS * kKUnit, pb += 2 * UNITS * kKUnit, px += 2 * UNITS * kKUnit;
 #pragma unroll
     for (int u = 0; u < UNITS; ++u) {
-      float(&first)[4] = acc.d[u & 1][0];
-      float(&second)[4] = acc.d[u & 1][1];
-      const uint4 a0 = va[u][0], x0 = vx[u][0];
+      // (rows 8..15 of the two forms without them are not summed)
+      constexpr int NSUM = FORM == FORM_FULL || FORM == FORM_ROWS8 ? 4 : 2;
+      float first[4], second[4];
       if (FORM == FORM_ROWS4) {
-        mma_k16<T>(first, a0.x, 0u, a0.y, 0u, x0.x, x0.y);
-        mma_k16<T>(first, a0.z, 0u, a0.w, 0u, x0.z, x0.w);
+        mma_k32<T>(first, va[u][0], zero, vx[u][0]);
       } else if (FORM == FORM_ROWS8) {
-        const uint4 a1 = va[u][NA - 1];
-        mma_k16<T>(first, a0.x, a1.x, a0.y, a1.y, x0.x, x0.y);
-        mma_k16<T>(first, a0.z, a1.z, a0.w, a1.w, x0.z, x0.w);
+        mma_k32<T>(first, va[u][0], va[u][NA - 1], vx[u][0]);
       } else {
-        const uint4 a1 = va[u][NA - 1], x1 = vx[u][NX - 1];
-        const uint4 b0 = NB ? vb[u][0] : zero, b1 = NB ? vb[u][NB ? NB - 1 : 0] : zero;
-        mma_k16<T>(first, a0.x, b0.x, a0.y, b0.y, x0.x, x0.y);
-        mma_k16<T>(first, a0.z, b0.z, a0.w, b0.w, x0.z, x0.w);
-        mma_k16<T>(second, a1.x, b1.x, a1.y, b1.y, x1.x, x1.y);
-        mma_k16<T>(second, a1.z, b1.z, a1.w, b1.w, x1.z, x1.w);
+        mma_k32<T>(first, va[u][0], NB ? vb[u][0] : zero, vx[u][0]);
+        mma_k32<T>(second, va[u][NA - 1], NB ? vb[u][NB ? NB - 1 : 0] : zero, vx[u][NX - 1]);
+      }
+#pragma unroll
+      for (int i = 0; i < NSUM; ++i) {
+        acc.d[0][i] += first[i];
+        if (!SPLIT) acc.d[1][i] += second[i];
       }
     }
   }
@@ -812,8 +811,8 @@ __device__ __forceinline__ void shrink_partials(const ShrinkAcc& acc, float (&ou
   float first[4], second[4];
 #pragma unroll
   for (int i = 0; i < 4; ++i) {
-    first[i] = acc.d[0][0][i] + acc.d[1][0][i];
-    second[i] = acc.d[0][1][i] + acc.d[1][1][i];
+    first[i] = acc.d[0][i];
+    second[i] = acc.d[1][i];
   }
   if (FORM == FORM_ROWS4) {  // the second fragment's sums sit four rows and four columns on: eighteen lanes
 #pragma unroll

@@ -5,7 +5,10 @@
 // descriptor layouts; here the operands of one instruction are 16 scattered rows against a handful of tokens that sit
 // in a stage as the bulk copies left them, and the consumers are bound by the instructions they issue, not by the
 // tensor pipe: one mma replaces 64 fused multiply-adds per lane.  Against 64-bit results the error of both forms is that
-// of the 16-bit outputs (2.2e-4 to 2.6e-4 in fp16, 1.9e-3 in bf16 on every batch measured, the same to two digits).
+// of the 16-bit outputs (2.2e-4 to 2.6e-4 in fp16, 1.9e-3 in bf16 on every batch measured).  Chains are short (32 values of
+// k, mma_k32), so that the FP32 sums behind them are no worse either: intermediates of fp16 batches that are not the
+// nearest value to the 64-bit sum, per thousand at hidden 4096 / 5120 / 8192: FMA 0.8 / 0.9 / 0.9, whole rows in one
+// accumulator 1.1 / 1.3 / 1.6, now 0.7 / 0.7 / 0.8.
 //
 // The dot product's order over k is free, so a fragment takes its k values where they lie: lane (g, t) = (lane / 4,
 // lane % 4) loads whole 16-byte vectors of its row and the token operand is loaded the same way, which makes both
@@ -36,6 +39,33 @@ __device__ __forceinline__ void mma_k16<__nv_bfloat16>(float (&d)[4], uint32_t a
       "%3};"
       : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3])
       : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
+}
+// d = a * b: the first of a chain.
+template <typename T>
+__device__ __forceinline__ void mma_k16_first(float (&d)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0,
+                                              uint32_t b1);
+template <>
+__device__ __forceinline__ void mma_k16_first<__half>(float (&d)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3,
+                                                      uint32_t b0, uint32_t b1) {
+  asm("mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%10, %10, %10, "
+      "%10};"
+      : "=f"(d[0]), "=f"(d[1]), "=f"(d[2]), "=f"(d[3])
+      : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1), "f"(0.f));
+}
+template <>
+__device__ __forceinline__ void mma_k16_first<__nv_bfloat16>(float (&d)[4], uint32_t a0, uint32_t a1, uint32_t a2,
+                                                             uint32_t a3, uint32_t b0, uint32_t b1) {
+  asm("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%10, %10, %10, "
+      "%10};"
+      : "=f"(d[0]), "=f"(d[1]), "=f"(d[2]), "=f"(d[3])
+      : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1), "f"(0.f));
+}
+// The 32 values of k that a 16-byte vector per lane holds, from zero: u, v = this lane's vectors of rows g and g + 8, b = of
+// column g.  Longer sums add such results with additions of their own: an mma truncates what it adds to its accumulator.
+template <typename T>
+__device__ __forceinline__ void mma_k32(float (&d)[4], const uint4& u, const uint4& v, const uint4& b) {
+  mma_k16_first<T>(d, u.x, v.x, u.y, v.y, b.x, b.y);
+  mma_k16<T>(d, u.z, v.z, u.w, v.w, b.z, b.w);
 }
 // The same with k = 8: a0 = row g, a1 = row g + 8, b0 = column g (two k values each).
 template <typename T>
@@ -118,6 +148,7 @@ __device__ __forceinline__ int expand_out(int cw, int gr, int g) {
 template <int R>
 struct DeltaFrag {
   uint32_t w[R <= 8 ? 1 : R / 8];
+  __device__ __forceinline__ uint4 vec(int i) const { return make_uint4(w[4 * i], w[4 * i + 1], w[4 * i + 2], w[4 * i + 3]); }
 };
 template <typename T, int R>
 __device__ __forceinline__ DeltaFrag<R> load_delta_frag(const T* ds, int tok, int t) {
@@ -150,14 +181,13 @@ __device__ __forceinline__ void expand_block_pair(float (&d)[4], const T* bs, co
   if constexpr (R == 16) {
     const uint2 u = *reinterpret_cast<const uint2*>(bs + o0 * 16 + 4 * t);
     const uint2 v = *reinterpret_cast<const uint2*>(bs + o1 * 16 + 4 * t);
-    mma_k16<T>(d, u.x, v.x, u.y, v.y, f.w[0], f.w[1]);
+    mma_k16_first<T>(d, u.x, v.x, u.y, v.y, f.w[0], f.w[1]);
   } else {
     static_assert(R >= 32, "rank 8 has its own loads");
     if constexpr (R == 32) {
       const uint4 u = *reinterpret_cast<const uint4*>(bs + o0 * 32 + 8 * t);
       const uint4 v = *reinterpret_cast<const uint4*>(bs + o1 * 32 + 8 * t);
-      mma_k16<T>(d, u.x, v.x, u.y, v.y, f.w[0], f.w[1]);
-      mma_k16<T>(d, u.z, v.z, u.w, v.w, f.w[2], f.w[3]);
+      mma_k32<T>(d, u, v, f.vec(0));
     } else {
       const bool odd = g & 1;
 #pragma unroll
@@ -169,10 +199,17 @@ __device__ __forceinline__ void expand_block_pair(float (&d)[4], const T* bs, co
         const uint4 wa = *reinterpret_cast<const uint4*>(bs + o1 * R + 8 * va);
         const uint4 wb = *reinterpret_cast<const uint4*>(bs + o1 * R + 8 * vb);
         const uint4 u0 = odd ? ub : ua, u1 = odd ? ua : ub, v0 = odd ? wb : wa, v1 = odd ? wa : wb;
-        mma_k16<T>(d, u0.x, v0.x, u0.y, v0.y, f.w[4 * i], f.w[4 * i + 1]);
-        mma_k16<T>(d, u0.z, v0.z, u0.w, v0.w, f.w[4 * i + 2], f.w[4 * i + 3]);
-        mma_k16<T>(d, u1.x, v1.x, u1.y, v1.y, f.w[4 * i + 4], f.w[4 * i + 5]);
-        mma_k16<T>(d, u1.z, v1.z, u1.w, v1.w, f.w[4 * i + 6], f.w[4 * i + 7]);
+        float e[4];
+        if (i == 0) {
+          mma_k32<T>(d, u0, v0, f.vec(0));
+        } else {
+          mma_k32<T>(e, u0, v0, f.vec(i));
+#pragma unroll
+          for (int q = 0; q < 4; ++q) d[q] += e[q];
+        }
+        mma_k32<T>(e, u1, v1, f.vec(i + 1));
+#pragma unroll
+        for (int q = 0; q < 4; ++q) d[q] += e[q];
       }
     }
   }
@@ -206,7 +243,7 @@ __device__ __forceinline__ void expand_group(float (&acc)[ExpandShape<R, PAIRED>
   } else {
 #pragma unroll
     for (int j = 0; j < S::NBLK / 2; ++j) {
-      float d[4] = {0.f, 0.f, 0.f, 0.f};
+      float d[4];
       expand_block_pair<T, R, PAIRED>(d, bs, f, cw, gr, j, nout, g, t);
       acc[2 * j][0] = d[0], acc[2 * j][1] = d[1];
       acc[2 * j + 1][0] = d[2], acc[2 * j + 1][1] = d[3];
