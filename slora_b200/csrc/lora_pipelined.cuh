@@ -749,61 +749,78 @@ __device__ __forceinline__ int shrink_form(int rows_per_item, int nrows, int n) 
   return nrows > 4 ? FORM_ROWS8 : FORM_ROWS4;
 }
 
-// Lane (g, t) reads 16-byte vector t of the 64 bytes of a row or token; rows and tokens beyond the real counts, and what
-// lies beyond the rows' end (rows end anywhere on a multiple of eight elements), are zero.  A stage starts at a whole
-// unit.  The loads of a round are issued before its first mma: the warp has nothing else to hide their latency with.
+// Lane (g, t) reads 16-byte vector t of the 64 bytes of a row or token; lanes beyond the real rows and tokens repeat the last
+// one (what they compute is in rows and columns that nobody reads), and in the last round of a row (END) what lies beyond
+// its end is zero: rows end anywhere on a multiple of eight elements.  A stage starts at a whole unit.  The loads of a
+// round are issued before its first mma: the warp has nothing else to hide their latency with.  (A round of two units:
+// with four or eight an item of four rows and one token took 1 to 4 % longer.  Checks of row, token and end at every load
+// instead: 1160 cycles an item of 4096 elements against 1050 and, in batches of single tokens, where two stages a CTA are
+// all that is in flight, 4 to 6 % of the launch.)
+constexpr int kRoundUnits = 2;
+template <int FORM>
+struct ShrinkShape {
+  static constexpr bool SPLIT = FORM == FORM_ROWS8 || FORM == FORM_ROWS4;
+  static constexpr int NA = FORM == FORM_ROWS4 ? 1 : 2, NB = FORM == FORM_FULL ? 2 : 0, NX = SPLIT ? 1 : 2;
+};
+template <typename T, int FORM, bool END>
+__device__ __forceinline__ void shrink_round(ShrinkAcc& acc, const unsigned char* pa, const unsigned char* pb,
+                                             const unsigned char* px, int left_a, int left_x) {
+  using S = ShrinkShape<FORM>;
+  const uint4 zero = make_uint4(0u, 0u, 0u, 0u);
+  uint4 va[kRoundUnits][S::NA], vb[kRoundUnits][S::NB ? S::NB : 1], vx[kRoundUnits][S::NX];
+#pragma unroll
+  for (int u = 0; u < kRoundUnits; ++u) {
+    const int k = u * kKUnit;
+    auto load = [&](const unsigned char* from, int h, int left) {
+      return !END || k + 32 * h < left ? *reinterpret_cast<const uint4*>(from + 2 * (k + 32 * h)) : zero;
+    };
+#pragma unroll
+    for (int h = 0; h < S::NA; ++h) va[u][h] = load(pa, h, left_a);
+#pragma unroll
+    for (int h = 0; h < S::NB; ++h) vb[u][h] = load(pb, h, left_a);
+#pragma unroll
+    for (int h = 0; h < S::NX; ++h) vx[u][h] = load(px, h, left_x);
+  }
+#pragma unroll
+  for (int u = 0; u < kRoundUnits; ++u) {
+    // (rows 8..15 of the two forms without them are not summed)
+    constexpr int NSUM = FORM == FORM_FULL || FORM == FORM_ROWS8 ? 4 : 2;
+    float first[4], second[4];
+    if (FORM == FORM_ROWS4) {
+      mma_k32<T>(first, va[u][0], zero, vx[u][0]);
+    } else if (FORM == FORM_ROWS8) {
+      mma_k32<T>(first, va[u][0], va[u][S::NA - 1], vx[u][0]);
+    } else {
+      mma_k32<T>(first, va[u][0], S::NB ? vb[u][0] : zero, vx[u][0]);
+      mma_k32<T>(second, va[u][S::NA - 1], S::NB ? vb[u][S::NB ? S::NB - 1 : 0] : zero, vx[u][S::NX - 1]);
+    }
+#pragma unroll
+    for (int i = 0; i < NSUM; ++i) {
+      acc.d[0][i] += first[i];
+      if (!S::SPLIT) acc.d[1][i] += second[i];
+    }
+  }
+}
 template <typename T, int FORM>
 __device__ __forceinline__ void shrink_accumulate(ShrinkAcc& acc, const unsigned char* st, int nrows, int n, int klen,
                                                   int cw, int lane) {
-  constexpr bool SPLIT = FORM == FORM_ROWS8 || FORM == FORM_ROWS4;
-  constexpr int UNITS = FORM == FORM_ROWS4 ? 4 : 2;  // of a round
-  constexpr int NA = FORM == FORM_ROWS4 ? 1 : 2, NB = FORM == FORM_FULL ? 2 : 0, NX = SPLIT ? 1 : 2;
+  using S = ShrinkShape<FORM>;
+  constexpr int ROUND = kRoundUnits * kKUnit;
   const int g = lane >> 2, t = lane & 3;
   const int bytes = klen * static_cast<int>(sizeof(T));
-  const uint4 zero = make_uint4(0u, 0u, 0u, 0u);
-  const int row = FORM == FORM_ROWS4 ? (g & 3) : g, tok = SPLIT ? (g & 3) : g;
+  const int row = FORM == FORM_ROWS4 ? (g & 3) : g, tok = S::SPLIT ? (g & 3) : g;
   const int ka = cw * (kKUnit / kConsumerWarps) + 8 * t + (FORM == FORM_ROWS4 ? 32 * (g >> 2) : 0);
-  const int kx = cw * (kKUnit / kConsumerWarps) + 8 * t + (SPLIT ? 32 * (g >> 2) : 0);
-  // the first element a lane may not read any more (0: none of them)
-  const int end_a = row < nrows ? klen - ka : 0, end_b = FORM == FORM_FULL && g + 8 < nrows ? klen - ka : 0,
-            end_x = tok < n ? klen - kx : 0;
-  const unsigned char* pa = st + chunk_at(row, bytes) + ka * 2;
-  const unsigned char* pb = st + chunk_at(g + 8, bytes) + ka * 2;
-  const unsigned char* px = st + chunk_at(nrows + tok, bytes) + kx * 2;
+  const int kx = cw * (kKUnit / kConsumerWarps) + 8 * t + (S::SPLIT ? 32 * (g >> 2) : 0);
+  const unsigned char* pa = st + chunk_at(min(row, nrows - 1), bytes) + ka * 2;
+  const unsigned char* pb = st + chunk_at(min(g + 8, nrows - 1), bytes) + ka * 2;
+  const unsigned char* px = st + chunk_at(nrows + min(tok, n - 1), bytes) + kx * 2;
+  int k0 = 0;
 #pragma unroll 1
-  for (int k0 = 0; k0 < klen; k0 += UNITS * kKUnit) {
-    uint4 va[UNITS][NA], vb[UNITS][NB ? NB : 1], vx[UNITS][NX];
-#pragma unroll
-    for (int u = 0; u < UNITS; ++u) {
-      const int k = u * kKUnit;
-#pragma unroll
-      for (int h = 0; h < NA; ++h) va[u][h] = k0 + k + 32 * h < end_a ? *reinterpret_cast<const uint4*>(pa + 2 * (k + 32 * h)) : zero;
-#pragma unroll
-      for (int h = 0; h < NB; ++h) vb[u][h] = k0 + k + 32 * h < end_b ? *reinterpret_cast<const uint4*>(pb + 2 * (k + 32 * h)) : zero;
-#pragma unroll
-      for (int h = 0; h < NX; ++h) vx[u][h] = k0 + k + 32 * h < end_x ? *reinterpret_cast<const uint4*>(px + 2 * (k + 32 * h)) : zero;
-    }
-    pa += 2 * UNITS * kKUnit, pb += 2 * UNITS * kKUnit, px += 2 * UNITS * kKUnit;
-#pragma unroll
-    for (int u = 0; u < UNITS; ++u) {
-      // (rows 8..15 of the two forms without them are not summed)
-      constexpr int NSUM = FORM == FORM_FULL || FORM == FORM_ROWS8 ? 4 : 2;
-      float first[4], second[4];
-      if (FORM == FORM_ROWS4) {
-        mma_k32<T>(first, va[u][0], zero, vx[u][0]);
-      } else if (FORM == FORM_ROWS8) {
-        mma_k32<T>(first, va[u][0], va[u][NA - 1], vx[u][0]);
-      } else {
-        mma_k32<T>(first, va[u][0], NB ? vb[u][0] : zero, vx[u][0]);
-        mma_k32<T>(second, va[u][NA - 1], NB ? vb[u][NB ? NB - 1 : 0] : zero, vx[u][NX - 1]);
-      }
-#pragma unroll
-      for (int i = 0; i < NSUM; ++i) {
-        acc.d[0][i] += first[i];
-        if (!SPLIT) acc.d[1][i] += second[i];
-      }
-    }
+  for (; k0 + ROUND <= klen; k0 += ROUND) {
+    shrink_round<T, FORM, false>(acc, pa, pb, px, 0, 0);
+    pa += 2 * ROUND, pb += 2 * ROUND, px += 2 * ROUND;
   }
+  if (k0 < klen) shrink_round<T, FORM, true>(acc, pa, pb, px, klen - k0 - ka, klen - k0 - kx);
 }
 // The warp's partial sums in C-fragment order: [0], [1] row g columns 2t, 2t + 1; [2], [3] row g + 8.
 template <int FORM>
