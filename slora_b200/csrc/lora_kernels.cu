@@ -546,16 +546,19 @@ int ensure_dyn_smem(K kernel, int which, size_t smem, size_t static_bytes = 0) {
 // factor a CTA only ever sees some of a tile's slot kinds, and where low-rank adapters leave the same kinds empty
 // every time (the second row block of a projection, say) the CTAs that see those would idle while the others do all
 // the work - e.g. 296 CTAs and 6 slots per tile: the odd CTAs would only get second row blocks.
-// Off unless SLORA_COPRIME_GRID=1: measured on one GPU only (a rank's kernels of the 13B-shaped batch under 8-way
-// tensor parallelism, emulated: 54.1 -> 51.6 us per layer; same-rank decode batches unchanged).
-int64_t pipe_grid(int64_t items, int per_tile, bool exact) {
-  static const bool coprime = [] {
+// `spread`: shrinks on one GPU, whose items of eight and sixteen rows leave fewer kinds a tile (64 rows wide, eight kinds a
+// projection: each of the 296 CTAs saw one of them): q,k,v of 256 single tokens over 1000 adapters of ranks 8 to 64 51.3 us with
+// 296 CTAs, 34.5 with 295 (39.9 with four rows an item and FMA consumers); adapters of one rank unchanged.  The other
+// launches only with SLORA_COPRIME_GRID=1: for the linked ones of tensor parallelism it is measured on one GPU only (a
+// rank's kernels of the 13B-shaped batch, emulated: 54.1 -> 51.6 us per layer).
+int64_t pipe_grid(int64_t items, int per_tile, bool exact, bool spread) {
+  static const bool everywhere = [] {
     const char* e = getenv("SLORA_COPRIME_GRID");
     return e && strcmp(e, "1") == 0;
   }();
   int64_t grid = static_cast<int64_t>(sm_count()) * kPipeCtasPerSm;
   if (items < grid) return items;
-  if (coprime && !exact && per_tile > 1) {
+  if ((spread || everywhere) && !exact && per_tile > 1) {
     auto gcd = [](int64_t a, int64_t b) {
       while (b) {
         const int64_t t = a % b;
@@ -713,7 +716,7 @@ int run_shrink(const TileSrc& src, const Tables& tb, const void* w, const void* 
     a.rows_per_row = make_fast_div(static_cast<uint32_t>(S / h_in));
     const int64_t items = static_cast<int64_t>(src.slots) * nproj * a.max_rb;
     const bool exact = (flags & SLORA_FLAG_EXACT_ITEMS) != 0 && src.mode == MODE_PLAN;
-    const int64_t grid = pipe_grid(items, nproj * a.max_rb, exact);
+    const int64_t grid = pipe_grid(items, nproj * a.max_rb, exact, tp == nullptr);
     const size_t smem = kShrinkRingBytes;
     auto go = [&](auto k, int which) {
       const int rc2 = ensure_dyn_smem(k, which, smem);
@@ -865,7 +868,7 @@ int run_expand(const TileSrc& src, const Tables& tb, const void* w, const void* 
     a.stride = make_fast_div(static_cast<uint32_t>(tb.pool_stride));
     const int64_t items = static_cast<int64_t>(src.slots) * a.chunk_begin[nproj];
     const bool exact = (flags & SLORA_FLAG_EXACT_ITEMS) != 0 && src.mode == MODE_PLAN;
-    const int64_t grid = pipe_grid(items, a.chunk_begin[nproj], exact);
+    const int64_t grid = pipe_grid(items, a.chunk_begin[nproj], exact, false);
     const size_t smem = exact ? kExpandRingBytes : kRingBytes;
     if (epi) {
       // the expand with rotary embedding / KV-pool scatter in its epilogue (lora_rope.cuh)
