@@ -13,7 +13,7 @@
 namespace slora {
 
 constexpr int kTileTokens = 8;  // tokens per tile (plan granularity)
-constexpr int kMaxRows = 4;     // adapter rows per shrink work item
+constexpr int kMaxRows = 4;     // adapter rows per work item of the simple shrink
 constexpr int kChunk = 8192;    // flat B elements per expand work item (16 KB)
 constexpr uint32_t kSpinLimit = 1u << 18;
 
@@ -156,7 +156,8 @@ struct ShrinkArgs {
   int max_rb;        // row blocks enumerated per (tile, projection)
   FastDiv per_tile;      // pipelined kernel: items enumerated per tile (padded enumeration)
   FastDiv rows_per_row;  // pipelined kernel: A rows per pool row
-  int rows_per_cta;  // <= kMaxRows
+  int rows_per_cta;  // adapter rows of an item: 4, 8 or 16 (pipelined kernel), <= kMaxRows (simple kernel), projections
+                     // of a CTA (tensor-core kernel)
   int tok_pass;      // simple kernel: tokens staged per pass
   int piece;         // simple kernel: elements per bulk copy
   int mma_stage_bytes;  // tensor-core kernel: bytes of one pipeline stage

@@ -58,9 +58,10 @@ constexpr int kShrinkRingBytes = SLORA_SHRINK_RING_KB * 1024;
 #define SLORA_EXPAND_RING_KB 104
 #endif
 // The expand's control block is 8 KB smaller (no reduction buffers): with 104 KB three of its ~34 KB stages (a B chunk
-// and one token's y segment and delta row) are in flight instead of two.  Used by the EXACT instantiation (long
-// launches over mixed ranks: measured -4 % on its q,k,v launch); the short launches of a same-rank decode batch
-// measured 2 % slower with it and keep kRingBytes.
+// and one token's y segment and delta row) are in flight instead of two.  Used by the EXACT instantiation (q,k,v expand
+// of the 13B-shaped batch 74.3 us with 96 KB, 72.6 with 104).  The padded one was given 96 KB when its consumers were
+// FMA loops and short launches 2 % slower with 104; with the present ones 104 would be the better size there too (rank-8
+// decode batch 9.3 -> 9.1 us, 77 tokens of mixed ranks 11.9 -> 11.3, 70B-shaped batch 55.4 -> 53.5).
 constexpr int kExpandRingBytes = SLORA_EXPAND_RING_KB * 1024;
 constexpr int kPipeCtasPerSm = 2;      // persistent CTAs per SM
 // Producer warps: the first resolves items and copies adapter rows, the second copies activations.
@@ -158,7 +159,7 @@ __device__ __forceinline__ bool tp_link_wait(const TpLink& tp, int lane) {
 // (shrink: all its columns have been written and fenced) or counts the exchange as done (expand: every CTA has read
 // its number).  One system-scope fence per CTA, by the thread that then bumps the arrival counter: the CTA barrier
 // before it orders every thread's stores before that fence, and a fence is cumulative.  (A fence by each of the CTA's
-// 288 threads, as this was first written, serialises in the memory system: measured, it cost more than the exchange
+// threads, as this was first written, serialises in the memory system: measured, it cost more than the exchange
 // itself.)  The expand's bookkeeping stays on this GPU and needs no system-scope fence at all.
 __device__ __forceinline__ void tp_link_finish(const TpLink& tp, bool is_shrink) {
   __shared__ int s_last;
@@ -360,11 +361,12 @@ __host__ __device__ __forceinline__ uint32_t round128(uint32_t v) { return (v + 
 // as ranks differ - the empty slots recur with the period of the slot grid.  With a plan the items are therefore
 // counted exactly: in closed form when every tile has the same rank (the plan's header says so), else through a
 // per-tile running count that the CTA builds in shared memory from the tile records (all threads fetch the
-// records, the producer warp scans the counts; before the grid-dependency wait: the plan is complete by then).  Without a plan, or with more tiles or items than the
-// control block holds, the padded enumeration stays.  The exact count costs the start of a launch a few hundred
-// nanoseconds (its arithmetic sits between the header and the first tile record), which a launch of ten
-// microseconds over same-rank adapters does not earn back: the kernels are therefore built both ways (EXACT) and
-// the caller, who can ask the plan what it holds (slora_plan_info), picks with SLORA_FLAG_EXACT_ITEMS.
+// records, the first producer warp scans the counts; before the grid-dependency wait: the plan is complete by then).
+// Without a plan, or with more tiles or items than the control block holds, the padded enumeration stays.  The exact
+// count costs the start of a launch a few hundred nanoseconds (its arithmetic sits between the header and the first
+// tile record), which a launch of ten microseconds over same-rank adapters does not earn back: the kernels are
+// therefore built both ways (EXACT) and the caller, who can ask the plan what it holds (slora_plan_info), picks with
+// SLORA_FLAG_EXACT_ITEMS.
 // ------------------------------------------------------------------------------------------------------------
 struct ItemMap {
   int mode = 0;      // 0 padded slots, 1 same count for every tile, 2 running count in PipeCtl::item_end
@@ -1261,7 +1263,7 @@ template <typename T, int R, int NT, bool INBAND>
 __device__ __forceinline__ void expand_stage(const T* bs, const int* m, T* y, int64_t y_stride, int lane, int cw,
                                              const T* dglobal, int64_t dglobal_stride, int32_t* status,
                                              volatile int* gave_up) {
-  using S = ExpandShape<R, false>;
+  using S = ExpandShape<R>;
   using K = TokenSplit<NT>;
   const int n = m[1], clen = m[4], obase = m[5];
   if (cw * (kPipeChunk / kConsumerWarps) >= clen) return;
@@ -1274,14 +1276,14 @@ __device__ __forceinline__ void expand_stage(const T* bs, const int* m, T* y, in
   const int g = lane >> 2, t = lane & 3;
   const DeltaFrag<R> f = load_delta_frag<T, R>(ds, K::column(g, n), t);
   const int tok0 = K::tok0(t);
-  const int x = expand_x<R, false>(g);
+  const int x = expand_x<R>(g);
   constexpr int ROUNDS = (S::NG + K::DUP - 1) / K::DUP;
 #pragma unroll 1
   for (int r = 0; r < ROUNDS; ++r) {
-    float acc[S::NBLK][2];
-    expand_round<T, R, false, NT>(acc, bs, f, cw, r, nout, lane);
+    float acc[S::VPL][2];
+    expand_round<T, R, NT>(acc, bs, f, cw, r, nout, lane);
     const int gr = r * K::DUP + K::di(t);
-    const int o = expand_out<R, false>(cw, gr, g);
+    const int o = expand_out<R>(cw, gr, g);
     const bool live = gr < S::NG && o < nout;
 #pragma unroll
     for (int c = 0; c < K::TPL; ++c) {

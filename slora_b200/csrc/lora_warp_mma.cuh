@@ -89,7 +89,7 @@ __device__ __forceinline__ void ldmatrix_x4(uint32_t (&r)[4], uint32_t addr) {
                : "memory");
 }
 
-// v[i] becomes v[i ^ x] for a lane value x below N (N = 1, 2, 4 or 8; selects, so that v stays in registers).
+// v[i] becomes v[i ^ x] for a lane value x below N (N = 2, 4 or 8; selects, so that v stays in registers).
 template <int N>
 __device__ __forceinline__ void xor_index(float (&v)[N], int x) {
 #pragma unroll
@@ -116,32 +116,25 @@ __device__ __forceinline__ void xor_index(float (&v)[N], int x) {
 // a 128-byte line in the other order.
 // Tokens are columns, and with fewer than eight of them the columns repeat them: all four lanes t of a row then hold
 // the same token's values, and each of them finishes (adds to y, stores) another group.
-//
-// PAIRED (rotary embedding): a group's blocks come in pairs, an element d < 64 of a head and its partner d + 64, which
-// the same lane holds: VPL counts pairs.
 // ------------------------------------------------------------------------------------------------------------
-template <int R, bool PAIRED>
+template <int R>
 struct ExpandShape {
   static constexpr int NOUT = 2048 / R;
-  static constexpr int UNITS = PAIRED ? NOUT / 2 : NOUT;  // outputs, or pairs of them
-  static constexpr int VPL = PAIRED ? (UNITS >= 128 ? 4 : (UNITS >= 64 ? 2 : 1)) : (R == 8 ? 8 : (R == 16 ? 4 : 2));
-  static constexpr int NG = UNITS / (8 * VPL);
-  static constexpr int NBLK = PAIRED ? 2 * VPL : VPL;  // blocks of eight rows per group (even)
+  static constexpr int VPL = R == 8 ? 8 : (R == 16 ? 4 : 2);
+  static constexpr int NG = NOUT / (8 * VPL);
 };
 
 // x(g): see above.
-template <int R, bool PAIRED>
+template <int R>
 __device__ __forceinline__ int expand_x(int g) {
-  if (PAIRED) return R == 8 ? (g >> 1) : (R == 16 ? ((g >> 1) & 1) : 0);
   return R == 8 ? g : (R == 16 ? (g & 3) : (R == 32 ? (g & 1) : 0));
 }
 
-// First output (inside the chunk) of the VPL this lane owns of group gr of warp cw; its pairs' second halves are 64 on.
-template <int R, bool PAIRED>
+// First output (inside the chunk) of the VPL this lane owns of group gr of warp cw.
+template <int R>
 __device__ __forceinline__ int expand_out(int cw, int gr, int g) {
-  using S = ExpandShape<R, PAIRED>;
-  const int unit = cw * S::UNITS + (gr * 8 + g) * S::VPL;
-  return PAIRED ? (unit >> 6) * 128 + (unit & 63) : unit;
+  using S = ExpandShape<R>;
+  return cw * S::NOUT + (gr * 8 + g) * S::VPL;
 }
 
 // The token operand: the delta rows of the tile's tokens, column g = token g (repeated below eight tokens).
@@ -170,14 +163,12 @@ __device__ __forceinline__ DeltaFrag<R> load_delta_frag(const T* ds, int tok, in
 
 // Row blocks 2j and 2j + 1 of group gr against the tokens: d[0..1] = this lane's output of block 2j for its two
 // columns, d[2..3] = that of block 2j + 1.  Rows past the chunk's nout outputs repeat the last one.
-template <typename T, int R, bool PAIRED>
+template <typename T, int R>
 __device__ __forceinline__ void expand_block_pair(float (&d)[4], const T* bs, const DeltaFrag<R>& f, int cw, int gr, int j,
                                                   int nout, int g, int t) {
-  const int base = expand_out<R, PAIRED>(cw, gr, g);
-  const int x = expand_x<R, PAIRED>(g);
-  const int q0 = PAIRED ? j : 2 * j, q1 = PAIRED ? j : 2 * j + 1;
-  const int o0 = min(base + (q0 ^ x), nout - 1);
-  const int o1 = min(base + (q1 ^ x) + (PAIRED ? 64 : 0), nout - 1);
+  const int base = expand_out<R>(cw, gr, g);
+  const int x = expand_x<R>(g);
+  const int o0 = min(base + ((2 * j) ^ x), nout - 1), o1 = min(base + ((2 * j + 1) ^ x), nout - 1);
   if constexpr (R == 16) {
     const uint2 u = *reinterpret_cast<const uint2*>(bs + o0 * 16 + 4 * t);
     const uint2 v = *reinterpret_cast<const uint2*>(bs + o1 * 16 + 4 * t);
@@ -216,20 +207,20 @@ __device__ __forceinline__ void expand_block_pair(float (&d)[4], const T* bs, co
 }
 
 // All of group gr: acc[b][c] = block b, column 2t + c of this lane.
-template <typename T, int R, bool PAIRED>
-__device__ __forceinline__ void expand_group(float (&acc)[ExpandShape<R, PAIRED>::NBLK][2], const T* bs,
+template <typename T, int R>
+__device__ __forceinline__ void expand_group(float (&acc)[ExpandShape<R>::VPL][2], const T* bs,
                                              const DeltaFrag<R>& f, int cw, int gr, int nout, int lane) {
-  using S = ExpandShape<R, PAIRED>;
+  using S = ExpandShape<R>;
   const int g = lane >> 2, t = lane & 3;
   if constexpr (R == 8) {
     // ldmatrix: four blocks at once, lane l points at row l % 8 of block l / 8
     const int rr = lane & 7, bi = lane >> 3;
-    const int base = expand_out<R, PAIRED>(cw, gr, rr);
-    const int x = expand_x<R, PAIRED>(rr);
+    const int base = expand_out<R>(cw, gr, rr);
+    const int x = expand_x<R>(rr);
 #pragma unroll
-    for (int j = 0; j < S::NBLK / 4; ++j) {
+    for (int j = 0; j < S::VPL / 4; ++j) {
       const int b = 4 * j + bi;
-      const int o = min(PAIRED ? base + ((b >> 1) ^ x) + (b & 1) * 64 : base + (b ^ x), nout - 1);
+      const int o = min(base + (b ^ x), nout - 1);
       uint32_t r[4];
       ldmatrix_x4(r, smem_u32(bs + o * 8));
 #pragma unroll
@@ -242,9 +233,9 @@ __device__ __forceinline__ void expand_group(float (&acc)[ExpandShape<R, PAIRED>
     }
   } else {
 #pragma unroll
-    for (int j = 0; j < S::NBLK / 2; ++j) {
+    for (int j = 0; j < S::VPL / 2; ++j) {
       float d[4];
-      expand_block_pair<T, R, PAIRED>(d, bs, f, cw, gr, j, nout, g, t);
+      expand_block_pair<T, R>(d, bs, f, cw, gr, j, nout, g, t);
       acc[2 * j][0] = d[0], acc[2 * j][1] = d[1];
       acc[2 * j + 1][0] = d[2], acc[2 * j + 1][1] = d[3];
     }
@@ -263,23 +254,23 @@ struct TokenSplit {
 };
 
 // Round `r` of a stage: after it acc holds the values of this lane's own group.
-template <typename T, int R, bool PAIRED, int NT>
-__device__ __forceinline__ void expand_round(float (&acc)[ExpandShape<R, PAIRED>::NBLK][2], const T* bs,
+template <typename T, int R, int NT>
+__device__ __forceinline__ void expand_round(float (&acc)[ExpandShape<R>::VPL][2], const T* bs,
                                              const DeltaFrag<R>& f, int cw, int r, int nout, int lane) {
-  using S = ExpandShape<R, PAIRED>;
+  using S = ExpandShape<R>;
   using K = TokenSplit<NT>;
   const int di = K::di(lane & 3);
 #pragma unroll
   for (int s = 0; s < K::DUP; ++s) {
     if (r * K::DUP + s >= S::NG) break;
     if (s == 0) {
-      expand_group<T, R, PAIRED>(acc, bs, f, cw, r * K::DUP, nout, lane);
+      expand_group<T, R>(acc, bs, f, cw, r * K::DUP, nout, lane);
     } else {
-      float other[S::NBLK][2];
-      expand_group<T, R, PAIRED>(other, bs, f, cw, r * K::DUP + s, nout, lane);
+      float other[S::VPL][2];
+      expand_group<T, R>(other, bs, f, cw, r * K::DUP + s, nout, lane);
       const bool mine = di == s;
 #pragma unroll
-      for (int b = 0; b < S::NBLK; ++b) {
+      for (int b = 0; b < S::VPL; ++b) {
 #pragma unroll
         for (int c = 0; c < K::TPL; ++c) acc[b][c] = mine ? other[b][c] : acc[b][c];
       }
@@ -287,7 +278,7 @@ __device__ __forceinline__ void expand_round(float (&acc)[ExpandShape<R, PAIRED>
   }
 }
 
-// N consecutive 16-bit values as one vector (N in 1, 2, 4, 8), and eight floats from / to them.
+// N consecutive 16-bit values as one vector (N in 2, 4, 8), and eight floats from / to them.
 template <typename T, int N>
 __device__ __forceinline__ void load_vec(float (&f)[N], const T* p) {
   if constexpr (N == 8) {
@@ -297,10 +288,8 @@ __device__ __forceinline__ void load_vec(float (&f)[N], const T* p) {
     T e[N];
     if constexpr (N == 4) {
       *reinterpret_cast<uint2*>(e) = *reinterpret_cast<const uint2*>(p);
-    } else if constexpr (N == 2) {
-      *reinterpret_cast<uint32_t*>(e) = *reinterpret_cast<const uint32_t*>(p);
     } else {
-      e[0] = *p;
+      *reinterpret_cast<uint32_t*>(e) = *reinterpret_cast<const uint32_t*>(p);
     }
 #pragma unroll
     for (int i = 0; i < N; ++i) f[i] = to_f32<T>(e[i]);
@@ -315,10 +304,8 @@ __device__ __forceinline__ void store_vec(T* p, const float (&f)[N]) {
     *reinterpret_cast<uint4*>(p) = *reinterpret_cast<const uint4*>(e);
   } else if constexpr (N == 4) {
     *reinterpret_cast<uint2*>(p) = *reinterpret_cast<const uint2*>(e);
-  } else if constexpr (N == 2) {
-    *reinterpret_cast<uint32_t*>(p) = *reinterpret_cast<const uint32_t*>(e);
   } else {
-    *p = e[0];
+    *reinterpret_cast<uint32_t*>(p) = *reinterpret_cast<const uint32_t*>(e);
   }
 }
 

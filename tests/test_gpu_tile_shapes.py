@@ -60,10 +60,24 @@ def test_rows_that_end_inside_a_unit(hidden, dtype):
         assert torch.equal(planned[p], single[p])
 
 
+def _few_at_a_time(wl, n=48):
+    """Per-token calls of `n` tokens: too few items for more than four rows each."""
+    w = wl.to(DEV)
+    ops = sl.LoraBatchOps(w.a_start, w.a_len, w.a_loc, w.a_scaling, w.pools_a, w.pools_b, wl.max_rank)
+    outs = [torch.zeros((wl.T, ho), dtype=wl.dtype, device=DEV) for _, ho in wl.proj_dims()]
+    for at in range(0, wl.T, n):
+        part = slice(at, at + n)
+        ops.prepare(w.ids[part], use_plan=False)
+        ops.lora_get_qkv(0, w.x_qkv[0][part], *(o[part] for o in outs[:3]))
+        ops.lora_get_o(0, w.x_o[0][part], outs[3][part])
+    torch.cuda.synchronize()
+    return outs
+
+
 @pytest.mark.parametrize("rows_case", ["16 rows", "8 rows", "8 rows, exact items"])
 def test_taller_items(rows_case):
-    """Batches large enough for items of sixteen and of eight rows; per-token calls of the same batch use four."""
-    if rows_case == "16 rows":      # 64 tokens an adapter: full tiles
+    """Batches large enough for items of sixteen and of eight rows, against calls of 48 tokens, whose items have four."""
+    if rows_case == "16 rows":      # 61 tokens an adapter: tiles of eight
         wl = build_workload(5, pool_rows=8192 + 512, n_adapters=33, decode_tokens=33 * 61, hidden=1032, h_kv=1032,
                             rank_choices=(64,))
         wl.ids = torch.arange(33 * 61) % 33
@@ -72,7 +86,7 @@ def test_taller_items(rows_case):
                             rank_choices=(64,) if rows_case == "8 rows" else (8, 16, 32, 64))
     ref = _oracle(wl)
     planned = _layer(wl, mixed_ranks=rows_case.endswith("items"), big_groups=False)
-    single = _layer(wl, use_plan=False)
+    single = _few_at_a_time(wl)
     for p in range(4):
         assert_parity(planned[p], ref[p], what=f"{rows_case} proj {p}")
         assert torch.equal(planned[p], single[p])
@@ -92,20 +106,6 @@ def test_ranks_that_fill_no_block():
         for t, a in enumerate(wl.ids.tolist()):
             r = wl.ranks[a]
             np.testing.assert_allclose(got[t, :r], ref[t, :r], rtol=2e-3, atol=2e-3)
-
-
-def _few_at_a_time(wl, n=48):
-    """Per-token calls of `n` tokens: too few items for more than four rows each."""
-    w = wl.to(DEV)
-    ops = sl.LoraBatchOps(w.a_start, w.a_len, w.a_loc, w.a_scaling, w.pools_a, w.pools_b, wl.max_rank)
-    outs = [torch.zeros((wl.T, ho), dtype=wl.dtype, device=DEV) for _, ho in wl.proj_dims()]
-    for at in range(0, wl.T, n):
-        part = slice(at, at + n)
-        ops.prepare(w.ids[part], use_plan=False)
-        ops.lora_get_qkv(0, w.x_qkv[0][part], *(o[part] for o in outs[:3]))
-        ops.lora_get_o(0, w.x_o[0][part], outs[3][part])
-    torch.cuda.synchronize()
-    return outs
 
 
 @pytest.mark.parametrize("exact", [False, True])
