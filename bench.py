@@ -367,9 +367,9 @@ def replay_median(step, replays, warmups=20):
 # adapters; traffic grows with the adapter rows and token rows a launch streams, as the algorithmic bytes do, so the
 # ratio carries over to the full launch).  Configurations without a capture print null.
 NCU_TRAFFIC_RATIO = {
-    (2, "expand"): ((32.76e6 + 0.016e6) / 38.93e6, "profiles/lora_pipe_kernels_cfg2_decode.md"),
-    (2, "shrink"): ((28.54e6 + 0.002e6) / 28.44e6, "profiles/lora_pipe_kernels_cfg2_decode.md"),
-    (4, "expand"): ((254.1e6 + 16.6e6) / 269.4e6, "profiles/lora_pipe_kernels_cfg4_mixed_ranks.md"),
+    (2, "expand"): ((32.77e6 + 0.010e6) / 38.93e6, "profiles/lora_pipe_kernels_cfg2_decode.md"),
+    (2, "shrink"): ((28.56e6 + 0.001e6) / 28.44e6, "profiles/lora_pipe_kernels_cfg2_decode.md"),
+    (4, "expand"): ((254.4e6 + 16.1e6) / 269.4e6, "profiles/lora_pipe_kernels_cfg4_mixed_ranks.md"),
     (4, "shrink"): ((243.4e6 + 4.4e6) / 243.1e6, "profiles/lora_pipe_kernels_cfg4_mixed_ranks.md"),
 }
 
